@@ -242,7 +242,8 @@ PyObject* sparse_mla(PyObject* const* a) {
     require(ws_o->scalar_type() == at::kFloat && ws_o->numel() >= rows * n_splits * heads * kDv, "split workspace: partials");
     require(ws_l && ws_l->scalar_type() == at::kFloat && ws_l->numel() >= rows * n_splits * heads, "split workspace: LSEs");
   } else if (n_splits > 1) {
-    n_splits = std::max<int64_t>(1, std::min<int64_t>(n_splits, MDC_STATIC_WS_MAX_SLOTS / (rows * heads)));
+    const int64_t per_split = std::max<int64_t>(1, rows * heads);   // (the launcher refuses an empty batch)
+    n_splits = std::max<int64_t>(1, std::min<int64_t>(n_splits, MDC_STATIC_WS_MAX_SLOTS / per_split));
     static_ws = n_splits > 1;
   }
   mdc_sparse_mla_params p{};
