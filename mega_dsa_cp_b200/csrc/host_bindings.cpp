@@ -114,7 +114,8 @@ PyObject* logits(PyObject* const* a) {
   const int64_t page = integer(a[14]), max_pages = bt.size(1);
   require(rows == T * kHeads, "query rows must be q_len * 64");
   if (row) require(rv->size(-1) == top_k && ri && ri->sizes() == rv->sizes() && rv->is_contiguous(), "row_topk tensors");
-  const int64_t n_chunks = (max_pages + bpc - 1) / bpc;
+  require(bpc >= 1, "blocks_per_chunk must be positive");
+  const int64_t n_chunks = max_pages / bpc + (max_pages % bpc != 0);
   for (const at::Tensor* t : {&kv, &q, &w, &bt}) require(t->is_cuda() && t->is_contiguous(), "inputs must be contiguous CUDA tensors");
   require(bt.scalar_type() == at::kInt && w.scalar_type() == at::kFloat, "block_table is int32, weights are float32");
   require(kv.size(1) == page * 64 + page * (mxfp4 ? 4 : 8), "page size does not match fmt/page_tokens");

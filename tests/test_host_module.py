@@ -31,3 +31,16 @@ def test_an_empty_batch_is_refused():
     o, lse = "torch.zeros(B, 1, H, 512, dtype=torch.bfloat16)", "torch.zeros(B, 1, H)"
     for splits in (1, 2):
         assert _error_of(MLA % dict(B=0, o=o, lse=lse, splits=splits)) == "MdcError"
+
+
+LOGITS = """
+from mega_dsa_cp_b200.tiles.logits import run_fp4_paged_mqa_logits
+B, pages = 2, 4
+run_fp4_paged_mqa_logits(torch.zeros(8, 4608, dtype=torch.uint8), torch.zeros(B, 64, 128, dtype=torch.bfloat16), None, torch.zeros(B, 64),
+                         torch.zeros(B, pages, dtype=torch.int32), torch.zeros(B, pages * 64), %d, fmt="nvfp4", page_tokens=64, stream=0)
+"""
+
+
+def test_chunks_of_no_pages_are_refused():
+    for pages_per_chunk in (0, -1):
+        assert _error_of(LOGITS % pages_per_chunk) == "AssertionError"
