@@ -220,14 +220,21 @@ PyObject* sparse_mla(PyObject* const* a) {
   require(q.dim() == 4, "q is (B, T, H, d_qk)");
   const int64_t B = q.size(0), T = q.size(1), heads = q.size(2), rows = B * T;
   require(kv.scalar_type() == q.scalar_type() && kv.is_contiguous() && q.is_contiguous(), "q and kv_cmp: one dtype, contiguous");
-  int64_t o_stride, dv = o.size(-1);   // elements between the rows of o
-  if (o.is_contiguous()) {
+  // elements between the rows of o, and from its first to behind its last
+  int64_t o_stride, room;
+  const int64_t dv = o.size(-1);
+  if (o.dim() == 4 && o.is_contiguous()) {
     o_stride = heads * dv;
+    room = o.numel();
+    require(room == rows * o_stride, "o is (B, T, H, 512)");
   } else {
     const at::Tensor o2 = o.dim() == 4 ? o.view({rows, heads, dv}) : o;
-    require(o2.stride(2) == 1 && o2.stride(1) == o2.size(2), "the heads of a row of o must be contiguous");
+    require(o2.dim() == 3 && o2.stride(2) == 1 && o2.stride(1) == o2.size(2), "the heads of a row of o must be contiguous");
     o_stride = o2.stride(0);
+    room = o2.size(0) > 0 ? (o2.size(0) - 1) * o_stride + o2.size(1) * o2.size(2) : 0;
   }
+  require(rows == 0 || (rows - 1) * o_stride + heads * kDv <= room, "o does not hold the output rows");
+  require(!lse || lse->numel() == rows * heads, "lse is (B, T, H)");
   // KV splits so that rows * heads / 64 * splits blocks roughly fill the SMs
   int64_t n_splits;
   if (a[12] == Py_None) {

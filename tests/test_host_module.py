@@ -8,29 +8,40 @@ import sys
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-def _error_of(body):
-    """Name of the exception that `body` raises in a fresh interpreter (a crash there fails the test, not the session)."""
-    code = "import sys\nsys.path.insert(0, %r)\nimport torch\ntry:\n" % ROOT
-    code += "".join("    " + line + "\n" for line in body.strip().splitlines())
-    code += "    print('NONE')\nexcept Exception as e:\n    print(type(e).__name__)\n"
+def _errors_of(bodies):
+    """Names of the exceptions that the pieces of code raise in a fresh interpreter (a crash there fails the test, not
+    the session)."""
+    code = "import sys\nsys.path.insert(0, %r)\nimport torch\n" % ROOT
+    for body in bodies:
+        code += "try:\n" + "".join("    " + line + "\n" for line in body.strip().splitlines())
+        code += "    print('NONE')\nexcept Exception as e:\n    print(type(e).__name__)\n"
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, (r.returncode, r.stderr[-1000:])
-    return r.stdout.split()[-1]
+    return r.stdout.split()
 
 
 MLA = """
 from mega_dsa_cp_b200.tiles.hca import run_sparse_mla
 B, H, D = %(B)s, 128, 576
 q, kv = torch.zeros(B, 1, H, D, dtype=torch.bfloat16), torch.zeros(4, 1, D, dtype=torch.bfloat16)
-pt, n = torch.zeros(B, 4, dtype=torch.int32), torch.zeros(B, dtype=torch.int32)
+pt, n = torch.zeros(B, 4, dtype=torch.int32), torch.zeros(0, dtype=torch.int32)   # (no lengths: the launcher refuses every call)
 run_sparse_mla(q, None, kv, None, pt, %(o)s, %(lse)s, n, None, None, 0.04, n_splits=%(splits)s, stream=0)
 """
+O, LSE = "torch.zeros(B, 1, H, 512, dtype=torch.bfloat16)", "torch.zeros(B, 1, H)"
 
 
 def test_an_empty_batch_is_refused():
-    o, lse = "torch.zeros(B, 1, H, 512, dtype=torch.bfloat16)", "torch.zeros(B, 1, H)"
-    for splits in (1, 2):
-        assert _error_of(MLA % dict(B=0, o=o, lse=lse, splits=splits)) == "MdcError"
+    assert _errors_of(MLA % dict(B=0, o=O, lse=LSE, splits=splits) for splits in (1, 2)) == ["MdcError"] * 2
+
+
+def test_outputs_that_do_not_hold_the_rows_are_refused():
+    fits = [(O, LSE), ("torch.zeros(3, H, 512)", "None"), ("torch.zeros(B, 2, H, 512)[:, :1]", LSE), ("torch.zeros(B, 1, H * 512)", LSE)]
+    assert _errors_of(MLA % dict(B=2, o=o, lse=l, splits=1) for o, l in fits) == ["MdcError"] * len(fits)   # (as far as the launcher)
+    small = [(o, LSE) for o in ("torch.zeros(1, 1, H, 512)", "torch.zeros(1, H, 512)", "torch.zeros(B, H // 2, 512)", "torch.zeros(B, H, 256)",
+                                "torch.zeros(B, 1, H, 256)", "torch.zeros(B, H * 512)", "torch.zeros(B, H, 1024)[:, :, :512]")]
+    small += [(O, "torch.zeros(1, 1, H)"), (O, "torch.zeros(B, 1, H // 2)")]
+    got = _errors_of(MLA % dict(B=2, o=o, lse=l, splits=1) for o, l in small)
+    assert all(e in ("AssertionError", "RuntimeError") for e in got), list(zip(small, got))
 
 
 LOGITS = """
@@ -42,5 +53,4 @@ run_fp4_paged_mqa_logits(torch.zeros(8, 4608, dtype=torch.uint8), torch.zeros(B,
 
 
 def test_chunks_of_no_pages_are_refused():
-    for pages_per_chunk in (0, -1):
-        assert _error_of(LOGITS % pages_per_chunk) == "AssertionError"
+    assert _errors_of(LOGITS % pages_per_chunk for pages_per_chunk in (0, -1)) == ["AssertionError"] * 2
