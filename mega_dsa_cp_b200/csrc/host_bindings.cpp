@@ -358,7 +358,9 @@ PyObject* compress_finalize(PyObject* const* a) {
   p.freqs = ptr<float>(&freqs);
   p.freq_rows = static_cast<int32_t>(freqs.size(0));
   p.norm_eps = static_cast<float>(real(a[8]));
-  p.inv_fp8_scale = static_cast<float>(1.0 / real(a[10]));
+  const double fp8_scale = real(a[10]);
+  if (fp8_scale == 0.0) fail(PyExc_ZeroDivisionError, "fp8_scale must not be zero");
+  p.inv_fp8_scale = static_cast<float>(1.0 / fp8_scale);
   p.attn_pool_dtype = pool.scalar_type() == at::kFloat8_e4m3fn ? MDC_DT_E4M3 : MDC_DT_BF16;
   p.attn_pool = pool.data_ptr();
   p.idx_pool = ptr<uint8_t>(get_tensor(st, "idx_pool"));

@@ -54,3 +54,18 @@ run_fp4_paged_mqa_logits(torch.zeros(8, 4608, dtype=torch.uint8), torch.zeros(B,
 
 def test_chunks_of_no_pages_are_refused():
     assert _errors_of(LOGITS % pages_per_chunk for pages_per_chunk in (0, -1)) == ["AssertionError"] * 2
+
+
+FINALIZE = """
+from mega_dsa_cp_b200.comm.buffers import alloc_arena
+from mega_dsa_cp_b200.events.symm import alloc_event_buffer
+from mega_dsa_cp_b200.tiles.compress import CompressorState, launch_finalize, stats_bytes
+st = CompressorState(1, 1, 0, 4, 0, device="cpu")   # (no entries: the launcher refuses every call)
+f = torch.zeros(512)
+launch_finalize(st, torch.zeros(1, dtype=torch.int32), alloc_arena({"stats": stats_bytes(4)}, 1, device="cpu"), "stats",
+                alloc_event_buffer(1, device="cpu"), 0, f, f, 1e-6, torch.zeros(4, 64), fp8_scale=%s, stream=0)
+"""
+
+
+def test_a_zero_fp8_scale_is_refused():
+    assert _errors_of(FINALIZE % scale for scale in ("0.02", "0.0")) == ["MdcError", "ZeroDivisionError"]
