@@ -288,22 +288,22 @@ PyObject* sparse_mla(PyObject* const* a) {
   return launch(static_ws ? entries.sparse_mla_static_ws : entries.sparse_mla, p, stream_of(a[15]));
 }
 
-// ---- compressor: the state, arena and event objects are read by attribute
-PyObject* get(PyObject* o, const char* name) {   // new reference, kept alive by its owner: the borrowed pointer is returned
-  PyObject* v = PyObject_GetAttrString(o, name);
-  if (!v) throw Failed{};
-  Py_DECREF(v);
-  return v;
+// ---- compressor: the state, arena and event objects are read by attribute, each held while it is read
+struct Ref {
+  PyObject* o;
+  explicit Ref(PyObject* x) : o(x) {
+    if (!o) throw Failed{};
+  }
+  Ref(const Ref&) = delete;
+  ~Ref() { Py_DECREF(o); }
+};
+Ref get(PyObject* o, const char* name) { return Ref(PyObject_GetAttrString(o, name)); }
+int64_t get_int(PyObject* o, const char* name) { return integer(get(o, name).o); }
+template <typename T = void>
+T* get_ptr(PyObject* o, const char* name) {
+  const Ref r = get(o, name);
+  return ptr<T>(tensor(r.o));
 }
-int64_t get_int(PyObject* o, const char* name) {
-  PyObject* v = PyObject_GetAttrString(o, name);
-  if (!v) throw Failed{};
-  const int64_t x = PyLong_AsLongLong(v);
-  Py_DECREF(v);
-  if (x == -1 && PyErr_Occurred()) throw Failed{};
-  return x;
-}
-const at::Tensor* get_tensor(PyObject* o, const char* name) { return tensor(get(o, name)); }
 
 void fill_compress(mdc_compress_params& p, PyObject* st, const at::Tensor& seq_len, PyObject* arena, PyObject* region, PyObject* events,
                    int64_t ev_base_id, int64_t phase, bool do_push, int64_t wait_budget_ns) {
@@ -314,24 +314,20 @@ void fill_compress(mdc_compress_params& p, PyObject* st, const at::Tensor& seq_l
   p.ratio = static_cast<int32_t>(get_int(st, "ratio"));
   p.phase = static_cast<int32_t>(phase);
   p.seq_len = ptr<int32_t>(&seq_len);
-  p.ring_attn = ptr<float>(get_tensor(st, "ring_attn"));
-  p.ring_idx = ptr<float>(get_tensor(st, "ring_idx"));
-  p.state = ptr<float>(get_tensor(st, "state"));
-  p.arena = mdc_peer_buffer{ptr(get_tensor(arena, "tensor")), ptr<int64_t>(get_tensor(arena, "offsets")),
+  p.ring_attn = get_ptr<float>(st, "ring_attn");
+  p.ring_idx = get_ptr<float>(st, "ring_idx");
+  p.state = get_ptr<float>(st, "state");
+  p.arena = mdc_peer_buffer{get_ptr(arena, "tensor"), get_ptr<int64_t>(arena, "offsets"),
                             static_cast<int32_t>(get_int(arena, "rank")), static_cast<int32_t>(get_int(arena, "world_size")),
                             get_int(arena, "mc_base")};
-  PyObject* off = PyDict_GetItemWithError(get(arena, "regions"), region);
-  if (!off) {
-    if (!PyErr_Occurred()) PyErr_SetObject(PyExc_KeyError, region);
-    throw Failed{};
-  }
-  p.stats_off = integer(off);
-  p.events = mdc_event_set{ptr(get_tensor(events, "tensor")), ptr<int64_t>(get_tensor(events, "offsets")),
+  const Ref regions = get(arena, "regions");
+  p.stats_off = integer(Ref(PyObject_GetItem(regions.o, region)).o);
+  p.events = mdc_event_set{get_ptr(events, "tensor"), get_ptr<int64_t>(events, "offsets"),
                            static_cast<int32_t>(get_int(events, "rank")), static_cast<int32_t>(get_int(events, "world_size"))};
   p.ev_base_id = static_cast<int32_t>(ev_base_id);
   p.do_push = do_push;
   p.wait_budget_ns = wait_budget_ns;
-  p.status = ptr<int32_t>(get_tensor(st, "status"));
+  p.status = get_ptr<int32_t>(st, "status");
 }
 
 // st, seq_len, new_attn, new_idx, ape_attn, ape_idx, arena, stats_region, events, ev_base_id, do_push, stream
@@ -352,7 +348,8 @@ PyObject* compress_finalize(PyObject* const* a) {
   PyObject* st = a[0];
   fill_compress(p, st, tensor_of(a[1]), a[2], a[3], a[4], integer(a[11]), integer(a[5]), true, integer(a[12]));
   const at::Tensor& freqs = tensor_of(a[9]);
-  const at::Tensor& pool = tensor_of(get(st, "attn_pool"));
+  const Ref attn_pool = get(st, "attn_pool");
+  const at::Tensor& pool = tensor_of(attn_pool.o);
   p.norm_w_attn = ptr<float>(tensor(a[6]));
   p.norm_w_idx = ptr<float>(tensor(a[7]));
   p.freqs = ptr<float>(&freqs);
@@ -363,13 +360,13 @@ PyObject* compress_finalize(PyObject* const* a) {
   p.inv_fp8_scale = static_cast<float>(1.0 / fp8_scale);
   p.attn_pool_dtype = pool.scalar_type() == at::kFloat8_e4m3fn ? MDC_DT_E4M3 : MDC_DT_BF16;
   p.attn_pool = pool.data_ptr();
-  p.idx_pool = ptr<uint8_t>(get_tensor(st, "idx_pool"));
+  p.idx_pool = get_ptr<uint8_t>(st, "idx_pool");
   p.idx_fmt = integer(a[14]) ? MDC_FMT_MXFP4 : MDC_FMT_NVFP4;
   p.idx_page_tokens = static_cast<int32_t>(get_int(st, "idx_page_tokens"));
   p.max_entries = static_cast<int32_t>(get_int(st, "max_entries"));
-  p.k_valid = ptr<int32_t>(get_tensor(st, "k_valid"));
-  p.dbg_attn = ptr<float>(get_tensor(st, "dbg_attn"));
-  p.dbg_idx = ptr<float>(get_tensor(st, "dbg_idx"));
+  p.k_valid = get_ptr<int32_t>(st, "k_valid");
+  p.dbg_attn = get_ptr<float>(st, "dbg_attn");
+  p.dbg_idx = get_ptr<float>(st, "dbg_idx");
   return launch(entries.compress_finalize, p, stream_of(a[13]));
 }
 

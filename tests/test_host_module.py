@@ -69,3 +69,14 @@ launch_finalize(st, torch.zeros(1, dtype=torch.int32), alloc_arena({"stats": sta
 
 def test_a_zero_fp8_scale_is_refused():
     assert _errors_of(FINALIZE % scale for scale in ("0.02", "0.0")) == ["MdcError", "ZeroDivisionError"]
+
+
+TEMPORARY = FINALIZE.replace("f = torch.zeros(512)", """f = torch.zeros(512)
+class Fresh(type(st)):   # attributes that exist only while they are read
+    attn_pool = property(lambda self: torch.zeros(1, 1, 512, dtype=torch.float8_e4m3fn), lambda self, v: None)
+    k_valid = property(lambda self: torch.zeros(1, dtype=torch.int32), lambda self, v: None)
+st = Fresh(1, 1, 0, 4, 0, device="cpu")""")
+
+
+def test_attributes_made_on_the_fly_are_held_while_they_are_read():
+    assert _errors_of([TEMPORARY % "0.02"] * 20) == ["MdcError"] * 20
