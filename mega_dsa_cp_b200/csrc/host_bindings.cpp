@@ -370,15 +370,22 @@ PyObject* compress_finalize(PyObject* const* a) {
   return launch(entries.compress_finalize, p, stream_of(a[13]));
 }
 
-// address of an mdc_mega_params (its owner keeps it alive), stream
+// address of an mdc_mega_params, address of the launch's mdc_layer_params (0: the one inside), stream, address and entries
+// of its trace, its wait budget (None: the one inside).  The block is read here, under the interpreter's lock: threads that
+// launch share it.
 PyObject* megakernel(PyObject* const* a) {
-  return launch(entries.megakernel, *reinterpret_cast<const mdc_mega_params*>(integer(a[0])), stream_of(a[1]));
+  mdc_mega_params p = *reinterpret_cast<const mdc_mega_params*>(integer(a[0]));
+  if (const int64_t layer = integer(a[1])) p.layer = *reinterpret_cast<const mdc_layer_params*>(layer);
+  p.trace = reinterpret_cast<unsigned long long*>(integer(a[3]));
+  p.trace_cap = static_cast<int32_t>(integer(a[4]));
+  if (a[5] != Py_None) p.wait_budget_ns = integer(a[5]);
+  return launch(entries.megakernel, p, stream_of(a[2]));
 }
 
 #define MDC_METHOD(name, n) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(entry<n, name>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {MDC_METHOD(bind, 1),          MDC_METHOD(logits, 22),        MDC_METHOD(merge_topk, 9),
                          MDC_METHOD(lse_merge, 6),     MDC_METHOD(sparse_mla, 18),    MDC_METHOD(compress_step, 12),
-                         MDC_METHOD(compress_finalize, 15), MDC_METHOD(megakernel, 2), {nullptr, nullptr, 0, nullptr}};
+                         MDC_METHOD(compress_finalize, 15), MDC_METHOD(megakernel, 6), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_mdc_host", "Host side of the tile runners", -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -91,13 +91,12 @@ def mega_params(ds: DeviceSchedule, events: EventBuffer, arena: SymmetricArena |
     return p
 
 
-def launch_params(p: N.MegaParams, layer: N.LayerParams | None = None, stream=None, trace: torch.Tensor | None = None) -> None:
-    """One launch with parameters of mega_params() (asynchronous)."""
-    if layer is not None:
-        p.layer = layer
-    p.trace = N.ptr(trace)
-    p.trace_cap = 0 if trace is None else (trace.numel() - 4) // 4
-    rc = N.host().megakernel(C.addressof(p), None if stream is None else N.stream_ptr(stream))
+def launch_params(p: N.MegaParams, layer: N.LayerParams | None = None, stream=None, trace: torch.Tensor | None = None,
+                  wait_budget_ns: int | None = None) -> None:
+    """One launch with parameters of mega_params() (asynchronous).  `p` is only read: what belongs to this launch (the
+    layer, the trace, a wait budget other than p's) goes into the launch's own copy."""
+    rc = N.host().megakernel(C.addressof(p), 0 if layer is None else C.addressof(layer), None if stream is None else N.stream_ptr(stream),
+                             0 if trace is None else trace.data_ptr(), 0 if trace is None else (trace.numel() - 4) // 4, wait_budget_ns)
     if rc < 0:
         N.check(rc, "mdc_megakernel_launch")
 

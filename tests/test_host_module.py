@@ -80,3 +80,19 @@ st = Fresh(1, 1, 0, 4, 0, device="cpu")""")
 
 def test_attributes_made_on_the_fly_are_held_while_they_are_read():
     assert _errors_of([TEMPORARY % "0.02"] * 20) == ["MdcError"] * 20
+
+
+def test_a_launch_leaves_the_shared_parameters_alone():
+    """Threads that launch one layer share its MegaParams: a launch takes a copy, its own layer, trace and budget in it."""
+    import pytest
+    import torch
+
+    from mega_dsa_cp_b200 import _native as N
+    from mega_dsa_cp_b200.schedule.device import launch_params
+
+    p = N.MegaParams(row_words=1, n_ctas=0, wait_budget_ns=7)   # (no blocks: the launcher refuses every call)
+    p.layer.B = 3
+    before, layer = bytes(p), N.LayerParams(B=5)
+    with pytest.raises(N.MdcError):
+        launch_params(p, layer, 0, torch.zeros(12, dtype=torch.int64), wait_budget_ns=9)
+    assert bytes(p) == before
