@@ -377,7 +377,7 @@ typedef struct {
   float* sel_v;                 /* (B, top_k) merged logits                      */
   int32_t* sel_i;               /* (B, top_k) global ids, identical on every rank */
   int32_t* sel_c;               /* (B,)                                          */
-  void* out;                    /* (ceil(B/cp), H, 512) merged attention output of the owned sequences: row b / cp for b % cp == rank */
+  void* out;                    /* (ceil(B/cp), H, 512) merged attention output of the owned sequences: row b / cp for b % cp == rank; 16 B aligned */
   float* out_lse;               /* (ceil(B/cp), H)                               */
   int32_t out_dtype;            /* MDC_DT_F32 | MDC_DT_BF16                      */
   /* two-level local merge: with l1_groups > 1 MERGE_L1A tasks first merge the chunk lists of one

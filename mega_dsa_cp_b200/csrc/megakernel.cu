@@ -893,6 +893,10 @@ static int layer_check(const mdc_mega_params& p) {
   }
   if (!L.sel_v || !L.sel_i || !L.sel_c || !L.out) return MDC_ERR_NULL;
   if (L.out_dtype != MDC_DT_F32 && L.out_dtype != MDC_DT_BF16) return MDC_ERR_BAD_FORMAT;
+  // written, and (histogram) read, in 16-byte pieces; the selection too where the ranks settle it together
+  const uintptr_t pieces = reinterpret_cast<uintptr_t>(L.out) | reinterpret_cast<uintptr_t>(L.thr_hist) |
+                           (L.thr_exact == 1 && L.cp > 1 ? reinterpret_cast<uintptr_t>(L.sel_v) | reinterpret_cast<uintptr_t>(L.sel_i) : 0);
+  if (pieces & 15) return MDC_ERR_BAD_ALIGN;
   if (L.l1_groups > 1 && (!L.mid_v || !L.mid_i || !L.mid_c)) return MDC_ERR_NULL;
   if (L.l1_groups < 0 || L.l1_groups > L.n_chunks) return MDC_ERR_BAD_SHAPE;
   if (L.cand_direct && L.cp > 1 && (L.l1_groups > 1 || L.cp * L.n_chunks > 256)) return MDC_ERR_BAD_SHAPE;  // the merge takes 256 lists

@@ -146,6 +146,29 @@ def test_megakernel_check_rejects_bad_layer_configurations():
         DsaDecodeLayer(4, cp=8, rank=0, attn_splits=4, device="cpu", n_ctas=8)
 
 
+def test_megakernel_check_refuses_misaligned_outputs():
+    """Buffers that the layer's tasks write or read in 16-byte pieces must start on such a boundary."""
+    from mega_dsa_cp_b200 import _native as N
+
+    chk = lambda p: N.lib().mdc_megakernel_check(C.byref(p))
+    A = 1 << 20
+    for at, want in ((A, 0), (A + 16, 0), (A + 2, -2), (A + 8, -2)):
+        p = _valid_mega_params(N)
+        p.layer.out = at
+        assert chk(p) == want, at - A
+    for name in ("out_lse", "sel_v", "sel_i", "sel_c"):       # written entry by entry with one rank
+        p = _valid_mega_params(N)
+        setattr(p.layer, name, A + 4)
+        assert chk(p) == 0, name
+    for name in ("sel_v", "sel_i", "thr_hist"):               # the selection published across ranks is copied in pieces
+        p = _valid_mega_params(N, cp=2)
+        p.layer.thr_hist = p.layer.thr_done = A
+        p.layer.thr_exact, p.layer.thr_ev_base, p.layer.thr_off, p.layer.cand_direct = 1, p.n_events, 4096, 1
+        assert chk(p) == 0
+        setattr(p.layer, name, A + 8)
+        assert chk(p) == -2, name
+
+
 def test_missing_library_fails_loudly(tmp_path):
     code = ("import os, sys; sys.path.insert(0, %r); os.environ['MDC_LIB_PATH'] = %r\n"
             "from mega_dsa_cp_b200 import _native\n"
