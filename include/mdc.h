@@ -51,7 +51,7 @@ extern "C" {
 
 /* query formats of the indexer */
 #define MDC_Q_FP4 0  /* (B, N, 64) packed E2M1 + (B, N*4) atom-ordered UE8M0 scales */
-#define MDC_Q_BF16 1 /* (B, N, 128) bf16                                             */
+#define MDC_Q_BF16 1 /* (B, N, 128) bf16, 16 B aligned                                           */
 
 /* element types of attention operands / partial outputs */
 #define MDC_DT_F32 0

@@ -107,7 +107,7 @@ int logits_check(const mdc_logits_params* p) {
     return MDC_ERR_NULL;
   }
   if (reinterpret_cast<uintptr_t>(p->kv_pages) & 15) return MDC_ERR_BAD_ALIGN;
-  if (reinterpret_cast<uintptr_t>(p->q) & 7) return MDC_ERR_BAD_ALIGN;
+  if (reinterpret_cast<uintptr_t>(p->q) & (p->q_fmt == MDC_Q_BF16 ? 15 : 7)) return MDC_ERR_BAD_ALIGN;   // (bf16 rows are read in 16-byte pieces)
   return MDC_OK;
 }
 

@@ -169,6 +169,18 @@ def test_megakernel_check_refuses_misaligned_outputs():
         assert chk(p) == -2, name
 
 
+def test_indexer_check_refuses_misaligned_queries():
+    """bf16 query rows are read in 16-byte pieces, FP4 rows in 4-byte ones (8 is what has been asked for)."""
+    from mega_dsa_cp_b200 import _native as N
+
+    A = 1 << 20
+    for q_fmt, at, good in ((N.Q_BF16, 0, True), (N.Q_BF16, 16, True), (N.Q_BF16, 8, False), (N.Q_FP4, 8, True), (N.Q_FP4, 4, False)):
+        p = N.LogitsParams(kv_pages=A, num_pages=4, page_tokens=64, fmt=N.FMT_NVFP4, q_fmt=q_fmt, q=A + at, q_sf=A, weights=A, block_table=A,
+                           max_pages=4, logits=A, logits_stride=256, B=1, q_len=1, heads=64, blocks_per_chunk=4, n_chunks=1, id_mul=1)
+        rc = N.lib().mdc_logits_fp4_smem_bytes(C.byref(p))
+        assert rc > 0 if good else rc == -2, (q_fmt, at, rc)
+
+
 def test_missing_library_fails_loudly(tmp_path):
     code = ("import os, sys; sys.path.insert(0, %r); os.environ['MDC_LIB_PATH'] = %r\n"
             "from mega_dsa_cp_b200 import _native\n"
