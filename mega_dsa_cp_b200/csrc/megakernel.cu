@@ -233,6 +233,9 @@ __device__ __noinline__ void op_kvwrite(const mdc_mega_params& p, int b) {
       uint4* dst = reinterpret_cast<uint4*>(static_cast<unsigned char*>(const_cast<void*>(L.mla.kv_cmp)) +
                                             (kv_row_base(L, b) + slot) * row_bytes);
       for (int i = tid; i < row_bytes / 16; i += kBlockThreads) dst[i] = src[i];
+      // The row's LOGITS tasks read the page by TMA in this same launch: these stores are made visible to the async proxy
+      // before the task's notify releases them (the tile's copy warp fences on its side).
+      if (tid < 32) fence_proxy_async_global();
       if (tid == 0) const_cast<int32_t*>(lp.seq_lens)[b] = slot + 1;
     }
   }

@@ -1283,6 +1283,7 @@ __device__ __forceinline__ int logits_tile(const mdc_logits_params& p, const CUt
       mbar_fence_init();
     }
     fence_proxy_async_smem();   // (the ring may have been the previous task's scratch)
+    if (!kAlone) fence_proxy_async_global();   // (a page may have been written by ordinary stores earlier in this launch)
     __syncwarp();
     int id = lane < n_pages ? bt[blk0 + lane] : -1;
     if (id >= p.num_pages) id = -1;

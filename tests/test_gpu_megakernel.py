@@ -516,3 +516,35 @@ def test_one_rank_selection_is_exact_on_tied_and_short_rows(S, K, n_ctas):
             assert torch.equal(layer.sel_i[b, :n].cpu(), ei), b
             assert torch.equal(layer.sel_v[b, :n].cpu().view(torch.int32), ev.view(torch.int32)), b
             assert torch.equal(layer.pt_local[b, :n].cpu(), ei + b * S) and int(layer.k_valid[b]) == 128 + n
+
+
+def test_every_new_token_is_scored_by_the_step_that_writes_it():
+    """KVWRITE stores the index record with ordinary stores and a LOGITS task of another block reads its page by TMA in
+    the same launch.  Each step's token points along the sum of the query heads, far above any other score, so every step
+    has to select it; the steps cross page boundaries, and the page's slot holds an all-zero record (score 0) before."""
+    from dsa_inputs import indexer_case
+    from mega_dsa_cp_b200.layer import DsaDecodeLayer, LayerInputs
+
+    B, S, K, P, DQK, steps = 6, 4096, 512, 64, 576, 80
+    case = indexer_case(B, S, P, "nvfp4", seed=51, shuffle=True)
+    start = torch.tensor([1500, 2000 + 63, 700, 3000, 1023, 2559], dtype=torch.int32)
+    for b in range(B):
+        for t in range(int(start[b]), int(start[b]) + steps):
+            pg = case["fused"][int(case["bt"][b, t // P])]
+            pg[(t % P) * 64:(t % P + 1) * 64] = 0
+    d = lambda t: t.to(DEV)
+    g = torch.Generator().manual_seed(52)
+    layer = DsaDecodeLayer(B, top_k=K, max_pages=S // P, blocks_per_chunk=16, kv_seq_stride=S, n_ctas=64, kvwrite=True)
+    lens = d(start)
+    layer.bind(LayerInputs(d(case["fused"]), d(case["bt"]), lens, d(case["q"]), torch.full((B, 64), 1 / 64, device=DEV),
+                           d((torch.randn(B, 1, 128, DQK, generator=g) * 0.5).bfloat16()),
+                           d((torch.randn(B * S, 1, DQK, generator=g) * 0.5).bfloat16())))
+    k_new = d(case["q_deq"].sum(1) / 8).contiguous()
+    layer.bind_kvwrite(k_new, torch.zeros(B, DQK, dtype=torch.bfloat16, device=DEV), lens.clone(), advance=True)
+    found = []
+    for s in range(steps):
+        layer.step()
+        found.append((layer.sel_i == (d(start) + s).view(B, 1)).any(1))
+    torch.cuda.synchronize()
+    layer.check_status()
+    assert bool(torch.stack(found).all()), torch.stack(found).logical_not().nonzero().tolist()
