@@ -363,6 +363,8 @@ int mdc_test_pingpong_launch(const mdc_pingpong_params* p, void* stream);
  *   inbox region: (B_owned, cp, H*512*2 + H*4) bytes, owner(b) = b % cp,
  *                 owned index b / cp: [H x 512 bf16 partial O][H f32 log2-LSE]  */
 #define MDC_THR_BINS 4096  /* bins of the row histogram: the upper 12 bits of the order-preserving u32 image of a score */
+#define MDC_THR_MAX_TOKENS 28544  /* chunks of more tokens (blocks_per_chunk * page_tokens) leave no room on chip for the histogram:
+                                   * their LOGITS tasks emit exact chunk lists, as without thr_hist, and the merges behind them select */
 
 typedef struct {
   int32_t cp, rank, B, top_k, H;

@@ -24,7 +24,7 @@ constexpr int kWarps = kBlockThreads / 32;
 __device__ inline void sync_workers() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
-__host__ __device__ inline int64_t align_up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
+__host__ __device__ constexpr int64_t align_up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
 
 // ------------------------------------------------------------------ status
 // A kernel that gives up on a wait (or finds an inconsistent input) records the

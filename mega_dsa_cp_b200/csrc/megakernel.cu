@@ -33,6 +33,15 @@ static_assert(kMegaThreads >= kMuThreads, "the block must hold the attention til
 constexpr int kStagedWords = 128;  // queue rows up to this length are staged in shared memory
 constexpr int kMegaTileSmem = MlaUmmaSmem<576>::kTotal > MlaSmem<576>::kTotal ? MlaUmmaSmem<576>::kTotal : MlaSmem<576>::kTotal;  // the largest tile
 
+// A row threshold keeps the histogram of the chunk's keys (16 KB) beside them.
+__device__ __host__ inline bool row_threshold_fits(const mdc_layer_params& L) {
+  return L.thr_hist && L.thr_done && L.logits.blocks_per_chunk <= MDC_THR_MAX_TOKENS / L.logits.page_tokens;
+}
+static_assert(logits_smem_layout<MDC_FMT_NVFP4, 64>(1, MDC_THR_MAX_TOKENS, true, true).total <= kMegaTileSmem &&
+                  logits_smem_layout<MDC_FMT_NVFP4, 128>(1, MDC_THR_MAX_TOKENS, true, true).total <= kMegaTileSmem &&
+                  logits_smem_layout<MDC_FMT_MXFP4, 128>(1, MDC_THR_MAX_TOKENS, true, true).total <= kMegaTileSmem,
+              "keys and histogram of the largest chunk");
+
 // The merge ops keep their scratch (MergeSmem) at the base of the tile's shared memory and stage the
 // lists behind it.
 constexpr int kMergeHdr = (static_cast<int>(sizeof(MergeSmem)) + 1023) / 1024 * 1024;
@@ -758,7 +767,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_kernel(const __grid_cons
           if (L.logits.page_tokens == 64) return op_logits<MDC_FMT_NVFP4, 64, T>(p, &pages, t.c0, t.c1, cur.phase, smem);
           return op_logits<MDC_FMT_NVFP4, 128, T>(p, &pages, t.c0, t.c1, cur.phase, smem);
         };
-        n = L.thr_hist && L.thr_done ? run(std::true_type{}) : run(std::false_type{});
+        n = row_threshold_fits(L) ? run(std::true_type{}) : run(std::false_type{});
         if (worker && n >= 0 && L.thr_exact == 4) op_row_fallback(p, t.c0, cur.phase, smem);
       }
         break;
@@ -914,8 +923,7 @@ static int layer_check(const mdc_mega_params& p) {
   if (static_cast<long long>(L.cp) * (L.attn_splits > 1 ? L.attn_splits : 1) > kLseMaxSlices) return MDC_ERR_TOO_LARGE;
   // the chunk's scores stay in shared memory: the tile's layout must fit the kernel's allocation
   const int ct = L.logits.blocks_per_chunk * L.logits.page_tokens;
-  const bool hist = L.thr_hist && L.thr_done;
-  if (hist && ct > 32768) return MDC_ERR_TOO_LARGE;
+  const bool hist = row_threshold_fits(L);
   int need;
   if (L.logits.fmt == MDC_FMT_MXFP4) need = logits_smem_layout<MDC_FMT_MXFP4, 128>(1, ct, true, hist).total;
   else if (L.logits.page_tokens == 64) need = logits_smem_layout<MDC_FMT_NVFP4, 64>(1, ct, true, hist).total;

@@ -110,8 +110,8 @@ struct LogitsSmem {
 };
 
 template <int FMT, int PAGE>
-__host__ __device__ inline LogitsSmem logits_smem_layout(int q_len, int chunk_tokens, bool fused, bool hist = false) {
-  LogitsSmem L;
+__host__ __device__ constexpr LogitsSmem logits_smem_layout(int q_len, int chunk_tokens, bool fused, bool hist = false) {
+  LogitsSmem L{};
   int off = 0;
   L.qb = off;  // [2 K-halves][N rows][128 B], swizzled; needs 1024 B alignment
   off += 2 * q_len * kIdxHeads * 128;

@@ -169,6 +169,34 @@ def test_megakernel_check_refuses_misaligned_outputs():
         assert chk(p) == -2, name
 
 
+@pytest.mark.parametrize("fmt,page,most", [("NVFP4", 64, 509), ("NVFP4", 128, 256), ("MXFP4", 128, 264)])
+def test_megakernel_check_takes_the_same_chunks_with_and_without_a_row_threshold(fmt, page, most):
+    """Up to the pages whose scores fit on chip; the threshold's histogram takes none of them away."""
+    from mega_dsa_cp_b200 import _native as N
+
+    for mode in (None, 0, 1, 4):
+        for pages, want in ((28544 // page, 0), (28544 // page + 1, 0), (most, 0), (most + 1, -6)):
+            p = _valid_mega_params(N, bpc=pages)
+            L = p.layer
+            L.logits.fmt, L.logits.page_tokens = getattr(N, "FMT_" + fmt), page
+            if mode is not None:
+                L.thr_hist = L.thr_done = 1 << 20
+                L.thr_exact, L.thr_ev_base, L.thr_off = mode, p.n_events, 4096
+            assert N.lib().mdc_megakernel_check(C.byref(p)) == want, (mode, pages)
+
+
+def test_layers_with_a_row_threshold_stay_within_its_chunks():
+    from mega_dsa_cp_b200.layer import DsaDecodeLayer
+
+    for page, fmt in ((64, "nvfp4"), (128, "nvfp4"), (128, "mxfp4")):
+        layer = DsaDecodeLayer(40, top_k=64, fmt=fmt, page_tokens=page, max_pages=131072 // page, blocks_per_chunk=32000 // page, n_ctas=148,
+                               device="cpu")
+        assert layer.bpc == 28544 // page and layer.n_chunks == 5
+        plain = DsaDecodeLayer(40, top_k=64, fmt=fmt, page_tokens=page, max_pages=131072 // page, blocks_per_chunk=32000 // page, n_ctas=148,
+                               device="cpu", row_threshold=False)
+        assert plain.bpc == 32000 // page
+
+
 def test_indexer_check_refuses_misaligned_queries():
     """bf16 query rows are read in 16-byte pieces, FP4 rows in 4-byte ones (8 is what has been asked for)."""
     from mega_dsa_cp_b200 import _native as N

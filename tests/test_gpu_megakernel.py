@@ -548,3 +548,39 @@ def test_every_new_token_is_scored_by_the_step_that_writes_it():
     torch.cuda.synchronize()
     layer.check_status()
     assert bool(torch.stack(found).all()), torch.stack(found).logical_not().nonzero().tolist()
+
+
+@pytest.mark.parametrize("capped", [True, False])
+@pytest.mark.parametrize("B,S,K", [(2, 63936, 2048), (3, 30080, 512)])
+def test_chunks_too_long_for_the_row_histogram(B, S, K, capped, monkeypatch):
+    """blocks_per_chunk beyond what leaves room for the row threshold's histogram: the layer takes chunks that fit;
+    a caller of the library that keeps them (the layer's limit lifted) gets the exact chunk lists and their merge."""
+    from dsa_inputs import indexer_case
+    from mega_dsa_cp_b200 import layer as layer_mod
+    from mega_dsa_cp_b200.tiles.logits import run_fp4_paged_mqa_logits
+    from oracle import dsa_oracle as orc
+
+    P, H, DQK = 64, 128, 576
+    pages = S // P
+    case = indexer_case(B, S, P, "nvfp4", seed=61)
+    g = torch.Generator().manual_seed(62)
+    seq = torch.tensor([S, S - 37, K - 5][:B], dtype=torch.int32)
+    if not capped:
+        monkeypatch.setattr(layer_mod, "THR_MAX_TOKENS", 1 << 30)
+    layer = layer_mod.DsaDecodeLayer(B, top_k=K, max_pages=pages, blocks_per_chunk=500, kv_seq_stride=S, out_dtype=torch.float32, n_ctas=2 * B - 1)
+    assert layer.row_exact == 4 and (layer.bpc * P <= 28544) == capped
+    d = lambda t: t.to(DEV)
+    layer.bind(layer_mod.LayerInputs(d(case["fused"]), d(case["bt"]), d(seq), d(case["q"]), d(case["w"]),
+                                     d((torch.randn(B, 1, H, DQK, generator=g) * 0.5).bfloat16()),
+                                     d((torch.randn(B * S, 1, DQK, generator=g) * 0.5).bfloat16())))
+    logits = torch.zeros(B, S, device=DEV)
+    run_fp4_paged_mqa_logits(d(case["fused"]), d(case["q"]), None, d(case["w"]), d(case["bt"]), logits, 16, fmt="nvfp4", page_tokens=P)
+    for _ in range(2):
+        layer.step()
+        torch.cuda.synchronize()
+        layer.check_status()
+        for b in range(B):
+            ev, ei = orc.local_topk_ref(logits[b].cpu(), 0, S, int(seq[b]), K, 1, 0)
+            n = int(layer.sel_c[b])
+            assert n == ei.numel() and torch.equal(layer.sel_i[b, :n].cpu(), ei), b
+            assert torch.equal(layer.sel_v[b, :n].cpu().view(torch.int32), ev.view(torch.int32)), b
