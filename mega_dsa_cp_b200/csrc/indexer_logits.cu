@@ -92,6 +92,7 @@ int logits_check(const mdc_logits_params* p) {
   if (p->fmt == MDC_FMT_MXFP4 && p->page_tokens != 128) return MDC_ERR_BAD_SHAPE;
   if (p->heads != kIdxHeads || (p->q_len != 1 && p->q_len != 2)) return MDC_ERR_BAD_SHAPE;
   if (p->num_pages < 1 || p->B < 1 || p->n_chunks < 1 || p->blocks_per_chunk < 1 || p->max_pages < 1) return MDC_ERR_BAD_SHAPE;
+  if (p->blocks_per_chunk > (1 << 20)) return MDC_ERR_TOO_LARGE;   // (far past what fits on chip; the sizes below are 32-bit)
   if (p->n_chunks > 65535 * 32 || p->B > 65535) return MDC_ERR_BAD_SHAPE;
   const bool fused = p->cand_v != nullptr && !p->row_v;
   if (p->row_v) {

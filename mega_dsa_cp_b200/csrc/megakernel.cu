@@ -35,7 +35,7 @@ constexpr int kMegaTileSmem = MlaUmmaSmem<576>::kTotal > MlaSmem<576>::kTotal ? 
 
 // A row threshold keeps the histogram of the chunk's keys (16 KB) beside them.
 __device__ __host__ inline bool row_threshold_fits(const mdc_layer_params& L) {
-  return L.thr_hist && L.thr_done && L.logits.blocks_per_chunk <= MDC_THR_MAX_TOKENS / L.logits.page_tokens;
+  return L.thr_hist && L.thr_done && L.logits.blocks_per_chunk * L.logits.page_tokens <= MDC_THR_MAX_TOKENS;
 }
 static_assert(logits_smem_layout<MDC_FMT_NVFP4, 64>(1, MDC_THR_MAX_TOKENS, true, true).total <= kMegaTileSmem &&
                   logits_smem_layout<MDC_FMT_NVFP4, 128>(1, MDC_THR_MAX_TOKENS, true, true).total <= kMegaTileSmem &&

@@ -169,6 +169,18 @@ def test_megakernel_check_refuses_misaligned_outputs():
         assert chk(p) == -2, name
 
 
+def test_indexer_check_refuses_chunks_whose_size_overflows():
+    from mega_dsa_cp_b200 import _native as N
+
+    A = 1 << 20
+    for pages in (1 << 24, 1 << 26, (1 << 31) - 1):
+        p = N.LogitsParams(kv_pages=A, num_pages=4, page_tokens=64, fmt=N.FMT_NVFP4, q_fmt=N.Q_BF16, q=A, weights=A, block_table=A, max_pages=4,
+                           cand_v=A, cand_i=A, cand_c=A, top_k=64, B=1, q_len=1, heads=64, blocks_per_chunk=pages, n_chunks=1, id_mul=1)
+        assert N.lib().mdc_logits_fp4_launch(C.byref(p), None) == -6, pages
+        q = _valid_mega_params(N, bpc=pages)
+        assert N.lib().mdc_megakernel_check(C.byref(q)) == -6, pages
+
+
 @pytest.mark.parametrize("fmt,page,most", [("NVFP4", 64, 509), ("NVFP4", 128, 256), ("MXFP4", 128, 264)])
 def test_megakernel_check_takes_the_same_chunks_with_and_without_a_row_threshold(fmt, page, most):
     """Up to the pages whose scores fit on chip; the threshold's histogram takes none of them away."""
