@@ -1,0 +1,108 @@
+"""Host side of the chunked prefill on the CPU: where a chunk's launches read and write.  The library's launches are
+replaced by a recorder, so nothing reaches a device."""
+
+import pytest
+import torch
+
+from mega_dsa_cp_b200 import _native as N
+from mega_dsa_cp_b200 import layer as layer_mod
+from mega_dsa_cp_b200 import prefill as prefill_mod
+
+H, DQK, K, TILE = 128, 576, 64, 2
+
+
+class _Lib:
+    """Stands in for libmdc.so: accepts the causal-length launch."""
+
+    def mdc_causal_lens_launch(self, *args):
+        return 0
+
+
+@pytest.fixture
+def launches(monkeypatch):
+    seen = []
+
+    def step(self, wait_budget_ns=0, stream=None, trace=None, _params=None):
+        L = N.LayerParams.from_buffer_copy(_params or self._params)
+        seen.append((self, L))
+        self.out.fill_(1.0)    # what a launch would leave in the layer's own buffers
+        self.out_lse.fill_(2.0)
+        self.sel_i.fill_(3)
+        self.sel_c.fill_(4)
+
+    monkeypatch.setattr(layer_mod.DsaDecodeLayer, "step", step)
+    monkeypatch.setattr(N, "lib", lambda: _Lib())
+    monkeypatch.setattr(N, "stream_ptr", lambda stream=None: 0)
+    return seen
+
+
+def _prefill(**kw):
+    args = dict(top_k=K, max_pages=4, blocks_per_chunk=2, n_ctas=16, device="cpu")
+    pf = prefill_mod.DsaPrefillChunk(TILE, **{**args, **kw})
+    pf.bind(torch.zeros(4, 4608, dtype=torch.uint8), torch.arange(4), torch.zeros(256, 1, DQK, dtype=torch.bfloat16))
+    return pf
+
+
+def _inputs(Tq):
+    return (torch.zeros(Tq, 64, 128, dtype=torch.bfloat16), torch.zeros(Tq, 64), torch.zeros(Tq, 1, H, DQK, dtype=torch.bfloat16),
+            torch.arange(Tq))
+
+
+def _results(Tq):
+    return dict(out=torch.zeros(Tq, H, 512, dtype=torch.bfloat16), out_lse=torch.zeros(Tq, H), sel_i=torch.zeros(Tq, K, dtype=torch.int32),
+                sel_c=torch.zeros(Tq, dtype=torch.int32))
+
+
+def _targets(launches, name):
+    return [getattr(L, name) for _, L in launches]
+
+
+def _offset(t, elements):
+    """A contiguous copy of t whose data starts `elements` elements behind a 16-byte boundary."""
+    buf = torch.zeros(t.numel() + elements, dtype=t.dtype)
+    return buf[elements:].view(t.shape)
+
+
+def test_results_that_fit_are_written_in_place(launches):
+    pf, res = _prefill(), _results(4)
+    pf.run(*_inputs(4), **res)
+    for name, t in res.items():
+        assert _targets(launches, name)[0] == t.data_ptr() and not t.any(), name
+
+
+@pytest.mark.parametrize("name,make", [
+    ("out", lambda t: t.float()),                                            # another type
+    ("out", lambda t: torch.zeros(4, H, 1024, dtype=t.dtype)[:, :, :512]),   # rows apart
+    ("out", lambda t: _offset(t, 1)),                                        # contiguous, but not 16-byte aligned
+    ("out_lse", lambda t: t.double()),
+    ("sel_i", lambda t: t.long()),
+    ("sel_i", lambda t: torch.zeros(4, 2 * K, dtype=t.dtype)[:, ::2]),
+    ("sel_c", lambda t: t.long()),
+])
+def test_other_results_are_copied(launches, name, make):
+    pf, res = _prefill(), _results(4)
+    res[name] = make(res[name])
+    pf.run(*_inputs(4), **res)
+    value = dict(out=1, out_lse=2, sel_i=3, sel_c=4)[name]
+    assert bool((res[name] == value).all())
+    assert all(L_target == getattr(layer, name).data_ptr() for (layer, _), L_target in zip(launches, _targets(launches, name)))
+
+
+def test_results_in_the_memory_of_an_input_are_copied(launches):
+    """A caller may let the output take the place of the attention query: it is written once the step is through."""
+    pf, res = _prefill(), _results(4)
+    q_idx, w, q_mla, pos = _inputs(4)
+    res["out"] = q_mla.view(-1)[:res["out"].numel()].view(res["out"].shape)
+    pf.run(q_idx, w, q_mla, pos, **res)
+    assert bool((res["out"] == 1).all()) and _targets(launches, "out")[0] == launches[0][0].out.data_ptr()
+
+
+@pytest.mark.parametrize("name,shape", [("out", (4, H, 256)), ("out", (3, H, 512)), ("out", (4, H // 2, 512)), ("out", (4 * H, 512)),
+                                        ("out_lse", (4, H // 2)), ("out_lse", (2, H)), ("sel_i", (4, K // 2)), ("sel_i", (1, K)),
+                                        ("sel_c", (2,)), ("sel_c", (4, 1))])
+def test_results_of_a_wrong_shape_are_refused(launches, name, shape):
+    pf, res = _prefill(), _results(4)
+    res[name] = torch.zeros(shape, dtype=res[name].dtype)
+    with pytest.raises((RuntimeError, IndexError)):
+        pf.run(*_inputs(4), **res)
+    assert all(getattr(L, name) == getattr(layer, name).data_ptr() for layer, L in launches)
