@@ -1,6 +1,9 @@
 """Host side of the chunked prefill on the CPU: where a chunk's launches read and write.  The library's launches are
 replaced by a recorder, so nothing reaches a device."""
 
+import gc
+import weakref
+
 import pytest
 import torch
 
@@ -106,3 +109,42 @@ def test_results_of_a_wrong_shape_are_refused(launches, name, shape):
     with pytest.raises((RuntimeError, IndexError)):
         pf.run(*_inputs(4), **res)
     assert all(getattr(L, name) == getattr(layer, name).data_ptr() for layer, L in launches)
+
+
+def test_every_call_reads_and_writes_its_own_tensors(launches):
+    """Another view at the same address, and a new tensor at a freed one's address, are other tensors."""
+    pf = _prefill()
+    q_idx, w, q_mla, pos = _inputs(4)
+    wide = torch.zeros(4, H, 1024, dtype=torch.bfloat16)
+    pf.run(q_idx, w, q_mla, pos, wide[:, :, :512])
+    assert bool((wide[:, :, :512] == 1).all()) and not wide[:, :, 512:].any()
+    wide.zero_()
+    every_other = wide.view(4, 2, H, 512)[:, 0]                        # same address and type, other strides
+    pf.run(q_idx, w, q_mla, pos, every_other)
+    assert bool((every_other == 1).all()) and not wide.view(4, 2, H, 512)[:, 1].any()
+    wide.zero_()
+    pf.run(q_idx, w, q_mla, pos, wide.view(8, H, 512)[:4])             # contiguous: in place
+    assert not wide.any() and launches[-1][1].out == wide.data_ptr()
+    for _ in range(3):
+        x, res = _inputs(4), _results(4)
+        x[1].fill_(1.0)
+        pf.run(*x, **res)
+        L = launches[-1][1]
+        assert (L.logits.q, L.logits.weights, L.mla.q, L.out) == (x[0].data_ptr(), x[1].data_ptr(), x[2].data_ptr(), res["out"].data_ptr())
+
+
+def test_tensors_of_a_call_are_not_kept(launches):
+    pf = _prefill()
+    x, res = _inputs(4), _results(4)
+    pf.run(*x, **res)
+    refs = [weakref.ref(t) for t in (*x, *res.values())]
+    del x, res
+    gc.collect()
+    assert not any(r() is not None for r in refs)
+
+
+def test_bind_wants_a_whole_row_of_the_page_table():
+    pf = _prefill()
+    for n in (1, 3, 8):
+        with pytest.raises(AssertionError):
+            pf.bind(torch.zeros(4, 4608, dtype=torch.uint8), torch.zeros(n, dtype=torch.int32), torch.zeros(256, 1, DQK, dtype=torch.bfloat16))
