@@ -148,3 +148,41 @@ def test_bind_wants_a_whole_row_of_the_page_table():
     for n in (1, 3, 8):
         with pytest.raises(AssertionError):
             pf.bind(torch.zeros(4, 4608, dtype=torch.uint8), torch.zeros(n, dtype=torch.int32), torch.zeros(256, 1, DQK, dtype=torch.bfloat16))
+
+
+@pytest.mark.parametrize("tile,Tqs", [(2, (2, 4, 2)), (1, (3, 1, 4)), (4, (4, 8))])
+def test_the_layers_are_built_with_the_object(launches, monkeypatch, tile, Tqs):
+    """A call of a size not seen before lays out nothing: every launch runs on a layer that the constructor built."""
+    monkeypatch.setattr(prefill_mod, "DsaDecodeLayer", _counted := _Counted(layer_mod.DsaDecodeLayer))
+    pf = prefill_mod.DsaPrefillChunk(tile, top_k=K, max_pages=4, blocks_per_chunk=2, n_ctas=16, device="cpu")
+    pf.bind(torch.zeros(4, 4608, dtype=torch.uint8), torch.arange(4), torch.zeros(256, 1, DQK, dtype=torch.bfloat16))
+    built = _counted.n
+    for Tq in Tqs:
+        del launches[:]
+        pf.run(*_inputs(Tq), **_results(Tq))
+        assert sum(L.B for _, L in launches) == Tq
+    assert _counted.n == built
+
+
+class _Counted:
+    def __init__(self, cls):
+        self.cls, self.n = cls, 0
+
+    def __call__(self, *a, **kw):
+        self.n += 1
+        return self.cls(*a, **kw)
+
+
+@pytest.mark.parametrize("tile", [1, 2, 3, 5, 8, 37])
+def test_chunks_of_every_size_are_covered_by_the_layers(launches, tile):
+    """Few launches, each of at most what fills the blocks, together exactly the chunk."""
+    pf = _prefill_of(tile, 148)
+    assert pf.max_tiles == 37 // tile and len(pf._layers) <= 17
+    for tiles in (1, 2, 3, 7, 8, 11, 12, 13, 17, 18, 23, 30, 31, 36, 37, 38, 75):
+        parts = list(pf._split(tiles))
+        assert sum(parts) == tiles and all(n in pf._layers for n in parts)
+        assert len(parts) <= -(-tiles // pf.max_tiles) + 2 and max(parts) <= pf.max_tiles
+
+
+def _prefill_of(tile, n_ctas):
+    return prefill_mod.DsaPrefillChunk(tile, top_k=K, max_pages=4, blocks_per_chunk=2, n_ctas=n_ctas, device="cpu")
