@@ -186,3 +186,9 @@ def test_chunks_of_every_size_are_covered_by_the_layers(launches, tile):
 
 def _prefill_of(tile, n_ctas):
     return prefill_mod.DsaPrefillChunk(tile, top_k=K, max_pages=4, blocks_per_chunk=2, n_ctas=n_ctas, device="cpu")
+
+
+def test_a_device_without_an_index_is_the_current_one(monkeypatch):
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    assert layer_mod.resolve_device("cuda") == torch.device("cuda", 3)
+    assert layer_mod.resolve_device("cuda:1") == torch.device("cuda", 1) and layer_mod.resolve_device("cpu") == torch.device("cpu")
