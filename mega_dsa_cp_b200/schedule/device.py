@@ -45,21 +45,30 @@ def task_offsets(row) -> list[int]:
     return offs
 
 
-def upload_schedule(schedule: Schedule, device="cuda", n_scalars: int = 8, dynamic_ctas: int | None = None) -> DeviceSchedule:
-    """dynamic_ctas: the schedule was generated for ONE queue (n_ctas = 1: all tasks of the rank in dependency
-    order); the kernel runs dynamic_ctas blocks that pull tasks from it with an atomic counter."""
+def host_words(schedule: Schedule) -> tuple[torch.Tensor, int]:
+    """What a schedule has on the device, as one int32 tensor on the host: queue rows, arities, scopes; and the row length."""
     flat, row = pack_queues(schedule)
-    n_ctas = len(schedule.queues)
-    i32 = lambda x: torch.tensor(x if len(x) else [0], dtype=torch.int32, device=device)
+    table = lambda x: x if len(x) else [0]
+    return torch.tensor(flat + table(schedule.arity) + table(schedule.scopes), dtype=torch.int32), row
+
+
+def upload_schedule(schedule: Schedule, device="cuda", n_scalars: int = 8, dynamic_ctas: int | None = None, words=None) -> DeviceSchedule:
+    """dynamic_ctas: the schedule was generated for ONE queue (n_ctas = 1: all tasks of the rank in dependency
+    order); the kernel runs dynamic_ctas blocks that pull tasks from it with an atomic counter.
+    words: host_words(schedule), from a caller that uploads one schedule several times."""
+    host, row = words or host_words(schedule)
+    n_ctas = queues = len(schedule.queues)
     dyn = {}
     if dynamic_ctas is not None:
         assert n_ctas == 1, "dynamic scheduling pulls from one shared queue: generate the schedule with n_ctas = 1"
-        offs = task_offsets(flat[:row])
-        dyn = dict(task_off=i32(offs), dyn_ctl=torch.zeros(2, dtype=torch.int32, device=device), n_tasks=len(offs))
+        offs = task_offsets(host[:row].tolist())
+        dyn = dict(task_off=torch.tensor(offs if offs else [0], dtype=torch.int32, device=device),
+                   dyn_ctl=torch.zeros(2, dtype=torch.int32, device=device), n_tasks=len(offs))
         n_ctas = dynamic_ctas
-    return DeviceSchedule(**dyn, 
-        queue=torch.tensor(flat, dtype=torch.int32, device=device).view(len(schedule.queues), row),
-        arity=i32(schedule.arity), scopes=i32(schedule.scopes),
+    sizes = [queues * row, max(1, len(schedule.arity)), max(1, len(schedule.scopes))]
+    queue, arity, scopes = host.to(device, copy=True).split(sizes)
+    return DeviceSchedule(**dyn,
+        queue=queue.view(queues, row), arity=arity, scopes=scopes,
         scalars=torch.zeros(n_scalars, dtype=torch.int64, device=device),
         phase_ctl=torch.zeros(1, dtype=torch.int64, device=device),
         n_ctas=n_ctas, row_words=row, n_events=schedule.n_events,
