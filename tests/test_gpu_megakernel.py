@@ -584,3 +584,45 @@ def test_chunks_too_long_for_the_row_histogram(B, S, K, capped, monkeypatch):
             n = int(layer.sel_c[b])
             assert n == ei.numel() and torch.equal(layer.sel_i[b, :n].cpu(), ei), b
             assert torch.equal(layer.sel_v[b, :n].cpu().view(torch.int32), ev.view(torch.int32)), b
+
+
+def test_merge_task_passes_on_what_the_chunk_tasks_published():
+    """thr_exact = 1 with one rank, the form of it that keeps a MERGE_L1 task per row (callers of the library; the layer
+    itself queues none): rows that the chunk tasks settled are left alone, tied ones merged."""
+    from dsa_inputs import indexer_case
+    from mega_dsa_cp_b200.comm.buffers import alloc_arena
+    from mega_dsa_cp_b200.events.symm import alloc_event_buffer
+    from mega_dsa_cp_b200.layer import DsaDecodeLayer, LayerInputs, arena_regions
+    from mega_dsa_cp_b200.schedule.device import mega_params
+    from mega_dsa_cp_b200.tiles.logits import run_fp4_paged_mqa_logits
+    from oracle import dsa_oracle as orc
+
+    B, S, K, P, H, DQK = 4, 8192, 1024, 64, 128, 576
+    case = indexer_case(B, S, P, "nvfp4", seed=81)
+    case["w"][0] = 0.0                                   # every score tied: falls back
+    g = torch.Generator().manual_seed(82)
+    seq = torch.tensor([S, S, S - 70, K // 3], dtype=torch.int32)
+    layer = DsaDecodeLayer(B, top_k=K, max_pages=S // P, blocks_per_chunk=32, kv_seq_stride=S, out_dtype=torch.float32, n_ctas=64, row_exact=False)
+    assert layer.n_chunks == 4 and layer.n_dag_events == layer.events.num_events
+    layer.row_exact = 1
+    layer.events = alloc_event_buffer(layer.n_dag_events + 2 * B, device=layer.device)
+    layer.arena = alloc_arena(arena_regions(B, 1, K, H, layer.attn_splits, thr_chunks=layer.n_chunks), layer.phases, device=layer.device)
+    layer._mega = mega_params(layer.dsched, layer.events, layer.arena, layer.status, device_phase=True)
+    d = lambda t: t.to(DEV)
+    layer.bind(LayerInputs(d(case["fused"]), d(case["bt"]), d(seq), d(case["q"]), d(case["w"]),
+                           d((torch.randn(B, 1, H, DQK, generator=g) * 0.5).bfloat16()),
+                           d((torch.randn(B * S, 1, DQK, generator=g) * 0.5).bfloat16())))
+    logits = torch.zeros(B, S, device=DEV)
+    run_fp4_paged_mqa_logits(d(case["fused"]), d(case["q"]), None, d(case["w"]), d(case["bt"]), logits, 16, fmt="nvfp4", page_tokens=P)
+    for _ in range(3):
+        layer.step()
+        torch.cuda.synchronize()
+        layer.check_status()
+        published = (layer.cand_c.view(B, -1) < 0).all(1).tolist()
+        assert published == [False, True, True, True]
+        for b in range(B):
+            ev, ei = orc.local_topk_ref(logits[b].cpu(), 0, S, int(seq[b]), K, 1, 0)
+            n = int(layer.sel_c[b])
+            assert n == ei.numel() and torch.equal(layer.sel_i[b, :n].cpu(), ei), b
+            assert torch.equal(layer.sel_v[b, :n].cpu().view(torch.int32), ev.view(torch.int32)), b
+            assert torch.equal(layer.pt_local[b, :n].cpu(), ei + b * S) and int(layer.k_valid[b]) == 128 + n
