@@ -327,13 +327,20 @@ inline int allow_dynamic_smem(int bytes) {
 }
 
 // A kernel that reads what the kernel before it on the stream writes is launched with launch_behind() and starts with
-// wait_for_predecessor(): its launch and its blocks' start overlap the predecessor, which calls let_successor_start()
-// first thing.  The wait ends when the predecessor's grid is complete and its writes are visible, as at an ordinary
-// kernel boundary; without the launch attribute it is no wait at all.  A successor's blocks are scheduled only once
-// every block of the predecessor runs or is done, so they cannot keep one from starting.
+// wait_for_predecessor(): its launch and its blocks' start overlap the predecessor's tail, or its whole run where that
+// calls let_successor_start() first thing.  The wait ends when the predecessor's grid is complete and its writes are
+// visible, as at an ordinary kernel boundary; without the launch attribute it is no wait at all.  A successor's blocks are
+// scheduled only once every block of the predecessor has called let_successor_start() or is done, so they cannot keep one
+// from starting.
 // 8 ranks' partials merged 4.6 -> 3.1 us, compressor step and finalize 12.3 -> 10.0, split attention of 3 queries 20.5 ->
 // 18.4 (16.8 with the attention kernel launched so too), chunk lists and their merge 32.1 -> 28.6, logits of 3 sequences
 // 8.2 -> 6.3, row top-k of 32 x 32768 41.0 -> 39.0, layer-step 1 x 4096 48.3 -> 44.8 and 8 x 131072 90.4 -> 88.4.
+//
+// The stand-alone indexer, the attention and the compressor kernels make the call: their chunk lists, split partials or
+// statistics are read by a small kernel right behind them.  The persistent kernel, the row top-k, the LSE merge, the list
+// merge and the split combine do not: with it layer-step 1 x 4096 45.8 -> 49.9 us (8 x 131072 unchanged), the LSE merge
+// 2.90 -> 3.28, row top-k 39.05 -> 39.46, list merge and combine unchanged (each called again and again; a successor's
+// waiting blocks share the SMs with the blocks they wait for).
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
