@@ -162,7 +162,7 @@ EXPORTS = [
 # the launchers the native host module calls, in the order of its table (csrc/host_bindings.cpp)
 _HOST_ENTRIES = ["mdc_logits_fp4_launch", "mdc_merge_topk_launch", "mdc_lse_merge_launch", "mdc_sparse_mla_launch",
                  "mdc_sparse_mla_launch_static_ws", "mdc_compress_step_launch", "mdc_compress_finalize_launch",
-                 "mdc_megakernel_launch"]
+                 "mdc_megakernel_launch", "mdc_causal_lens_launch"]
 
 
 def host():

@@ -23,6 +23,7 @@ struct Entries {
   int (*compress_step)(const mdc_compress_params*, void*);
   int (*compress_finalize)(const mdc_compress_params*, void*);
   int (*megakernel)(const mdc_mega_params*, void*);
+  int (*causal_lens)(const int64_t*, int32_t*, int32_t, int32_t, int32_t, void*);
 } entries;
 
 struct Failed {};   // a Python error has been set
@@ -382,10 +383,93 @@ PyObject* megakernel(PyObject* const* a) {
   return launch(entries.megakernel, p, stream_of(a[2]));
 }
 
+// ---- chunked prefill: addresses of a chunk's tensors in the launch parameters (prefill.py)
+struct Span {
+  uintptr_t lo, hi;
+};
+Span span_of(const at::Tensor& t) {   // the memory that a tensor may touch
+  if (t.is_contiguous()) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(t.data_ptr());
+    return {at, at + t.nbytes()};
+  }
+  const uintptr_t at = reinterpret_cast<uintptr_t>(t.storage().data());
+  return {at, at + t.storage().nbytes()};
+}
+PyObject* item(PyObject* tuple, Py_ssize_t i) {   // borrowed
+  PyObject* o = PyTuple_GetItem(tuple, i);
+  if (!o) throw Failed{};
+  return o;
+}
+constexpr int kResults = 4;   // out, out_lse (a row per owned query token), sel_i, sel_c (a row per query token)
+int64_t tokens_per_row(int result, int64_t cp) { return result < 2 ? cp : 1; }
+
+// positions (int64), lens (int32), cp, rank, stream
+PyObject* causal_lens(PyObject* const* a) {
+  const at::Tensor &pos = tensor_of(a[0]), &lens = tensor_of(a[1]);
+  require(pos.scalar_type() == at::kLong && lens.scalar_type() == at::kInt && pos.is_contiguous() && lens.is_contiguous() &&
+              pos.numel() == lens.numel(), "one int32 length per int64 position");
+  const int64_t cp = integer(a[2]), rank = integer(a[3]);
+  void* stream = stream_of(a[4]);
+  int rc;
+  Py_BEGIN_ALLOW_THREADS;
+  rc = entries.causal_lens(ptr<int64_t>(&pos), ptr<int32_t>(&lens), static_cast<int32_t>(pos.numel()), static_cast<int32_t>(cp),
+                           static_cast<int32_t>(rank), stream);
+  Py_END_ALLOW_THREADS;
+  return PyLong_FromLong(rc);
+}
+
+// The results that a chunk's launches can write straight into the caller's tensors, as a bit mask: rows of the shape, type
+// and device of the layer's own buffers, contiguous, on the 16-byte boundary that the kernels' stores need, and clear of the
+// memory of what the launches read.
+// tensors read, results (None: not asked for), the layer's own buffers, query tokens, cp
+PyObject* prefill_targets(PyObject* const* a) {
+  const Py_ssize_t n_reads = PyTuple_Size(a[0]);
+  if (n_reads < 0) throw Failed{};
+  const int64_t tokens = integer(a[3]), cp = integer(a[4]);
+  Span reads[8];
+  require(n_reads <= 8 && cp >= 1, "prefill_targets");
+  for (Py_ssize_t i = 0; i < n_reads; ++i) reads[i] = span_of(tensor_of(item(a[0], i)));
+  long mask = 0;
+  for (int r = 0; r < kResults; ++r) {
+    const at::Tensor *t = tensor(item(a[1], r)), &like = tensor_of(item(a[2], r));
+    if (!t || t->scalar_type() != like.scalar_type() || t->device() != like.device() || t->dim() != like.dim() || !t->is_contiguous()) continue;
+    if (t->sizes().slice(1) != like.sizes().slice(1) || t->size(0) < tokens / tokens_per_row(r, cp)) continue;
+    const Span s = span_of(*t);
+    bool clear = s.lo % 16 == 0;
+    for (Py_ssize_t i = 0; i < n_reads; ++i) clear = clear && (s.hi <= reads[i].lo || reads[i].hi <= s.lo);
+    if (clear) mask |= 1l << r;
+  }
+  return PyLong_FromLong(mask);
+}
+
+// address of the mdc_layer_params to fill, address of the layer's on its caches, causal lengths, q_idx (None: the queries
+// are staged), w_idx, q_mla, first query token of the launch, cp, results, mask of prefill_targets
+PyObject* prefill_fill(PyObject* const* a) {
+  mdc_layer_params& L = *reinterpret_cast<mdc_layer_params*>(integer(a[0]));
+  L = *reinterpret_cast<const mdc_layer_params*>(integer(a[1]));
+  const int64_t t0 = integer(a[6]), cp = integer(a[7]), mask = integer(a[9]);
+  auto row = [](const at::Tensor& t, int64_t i) { return static_cast<char*>(t.data_ptr()) + i * t.stride(0) * t.element_size(); };
+  L.logits.seq_lens = reinterpret_cast<int32_t*>(row(tensor_of(a[2]), t0));
+  if (const at::Tensor* q = tensor(a[3])) {
+    L.logits.q = row(*q, t0);
+    L.logits.weights = reinterpret_cast<float*>(row(tensor_of(a[4]), t0));
+    L.mla.q = row(tensor_of(a[5]), t0);
+  }
+  void* at[kResults] = {};
+  for (int r = 0; r < kResults; ++r)
+    if ((mask >> r) & 1) at[r] = row(tensor_of(item(a[8], r)), t0 / tokens_per_row(r, cp));
+  if (at[0]) L.out = at[0];
+  if (at[1]) L.out_lse = static_cast<float*>(at[1]);
+  if (at[2]) L.sel_i = static_cast<int32_t*>(at[2]);
+  if (at[3]) L.sel_c = static_cast<int32_t*>(at[3]);
+  Py_RETURN_NONE;
+}
+
 #define MDC_METHOD(name, n) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(entry<n, name>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {MDC_METHOD(bind, 1),          MDC_METHOD(logits, 22),        MDC_METHOD(merge_topk, 9),
                          MDC_METHOD(lse_merge, 6),     MDC_METHOD(sparse_mla, 18),    MDC_METHOD(compress_step, 12),
-                         MDC_METHOD(compress_finalize, 15), MDC_METHOD(megakernel, 6), {nullptr, nullptr, 0, nullptr}};
+                         MDC_METHOD(compress_finalize, 15), MDC_METHOD(megakernel, 6),
+                         MDC_METHOD(causal_lens, 5), MDC_METHOD(prefill_targets, 5), MDC_METHOD(prefill_fill, 10), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_mdc_host", "Host side of the tile runners", -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -1,5 +1,5 @@
-"""Host side of the chunked prefill on the CPU: where a chunk's launches read and write.  The library's launches are
-replaced by a recorder, so nothing reaches a device."""
+"""Host side of the chunked prefill on the CPU: where a chunk's launches read and write.  Both launches of a chunk are
+replaced (the step by a recorder), so nothing reaches a device."""
 
 import gc
 import weakref
@@ -12,13 +12,6 @@ from mega_dsa_cp_b200 import layer as layer_mod
 from mega_dsa_cp_b200 import prefill as prefill_mod
 
 H, DQK, K, TILE = 128, 576, 64, 2
-
-
-class _Lib:
-    """Stands in for libmdc.so: accepts the causal-length launch."""
-
-    def mdc_causal_lens_launch(self, *args):
-        return 0
 
 
 @pytest.fixture
@@ -34,8 +27,7 @@ def launches(monkeypatch):
         self.sel_c.fill_(4)
 
     monkeypatch.setattr(layer_mod.DsaDecodeLayer, "step", step)
-    monkeypatch.setattr(N, "lib", lambda: _Lib())
-    monkeypatch.setattr(N, "stream_ptr", lambda stream=None: 0)
+    monkeypatch.setattr(prefill_mod, "_device_lens", lambda *args: None)
     return seen
 
 
