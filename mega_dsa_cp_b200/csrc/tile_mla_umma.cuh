@@ -191,8 +191,9 @@ __device__ void mla_umma_tile(const mdc_sparse_mla_params& p, int r, int hb, int
   const int k_valid = min(max(p.k_valid[r], 0), kWinSlots + p.pt_cols * p.page_cmp);
   const int win_valid = p.win_valid ? min(max(p.win_valid[r], 0), kWinSlots) : 0;
   // Window slots in the tiles: the valid ones, no slots for the masked ones behind them.  e4m3 probabilities
-  // keep the masked slots: which slots share a tile decides how they round.
-  const int win = (win_valid > 0 && p.kv_win) ? (FP8 ? kWinSlots : win_valid) : 0;
+  // keep the masked slots: which slots share a tile decides how they round.  (k_valid counts the window's 128 slots: a row
+  // that ends before them has the window slots of its own tiles.)
+  const int win = (win_valid > 0 && p.kv_win) ? min(FP8 ? kWinSlots : win_valid, ceil_div(k_valid, kMuTile) * kMuTile) : 0;
   const int n_tiles_all = ceil_div(win + max(k_valid - kWinSlots, 0), kMuTile);
   const int per = ceil_div(n_tiles_all, n_splits);
   const int t_begin = split * per;

@@ -337,6 +337,30 @@ def test_sparse_mla_fp8_reference_mode():
         assert torch.allclose(l, rl, rtol=1e-3, atol=5e-3)
 
 
+@pytest.mark.parametrize("dtype,d_qk,H,splits", [(torch.bfloat16, 576, 128, 1), (torch.bfloat16, 512, 128, 2), (torch.bfloat16, 576, 64, 1),
+                                                 (torch.float8_e4m3fn, 512, 128, 1), (torch.float8_e4m3fn, 512, 64, 1)])
+def test_sparse_mla_rows_that_end_inside_the_window(dtype, d_qk, H, splits):
+    """k_valid counts the window's 128 slots; a row that ends before them attends the window slots of its own 64-slot
+    tiles only (none at all with k_valid 0, as idle rows of a batch have it), on every tile of this library."""
+    fp8 = dtype == torch.float8_e4m3fn
+    k_valid = [0, 1, 64, 65, 128, 130, 0, 40]
+    case = mla_case(len(k_valid), 1, H, d_qk, 300, [8] * len(k_valid), dtype=dtype, with_window=True, seed=15)
+    if fp8:
+        for k in ("q", "kv_cmp", "kv_win"):
+            case[k] = (case[k].float() * 40).clamp(-448, 448).to(dtype)
+    case["k_valid"] = torch.tensor(k_valid, dtype=torch.int32)
+    case["win_valid"] = torch.tensor([128, 128, 100, 70, 128, 30, 5, 20], dtype=torch.int32)
+    sink = torch.randn(H, generator=torch.Generator().manual_seed(2)) * 0.5 - 1.0
+    for s in (None, sink):
+        scale = 0.007 if fp8 else 1 / math.sqrt(d_qk)
+        o, l = _mla(case, s, scale, fp8_p=fp8, n_splits=splits)
+        ro, rl = mla_oracle(case, s, scale, fp8_p=fp8, online_tile=64)
+        fin = torch.isfinite(rl)
+        assert torch.equal(torch.isfinite(l), fin) and (l - rl)[fin].abs().max() < 1e-3
+        bad = ((o - ro).abs() > 2e-2 + (2e-2 * ro.abs() if fp8 else 0.0)).float().mean().item()
+        assert bad < (1e-3 if fp8 else 1e-9), bad
+
+
 def test_sparse_mla_bf16_partial_output_and_paged_pool():
     case = mla_case(2, 1, 128, 576, 40, [16 * 30, 16 * 11 + 5], seed=11, page_cmp=16)
     scale = 1.0 / math.sqrt(576)
