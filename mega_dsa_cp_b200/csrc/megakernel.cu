@@ -243,7 +243,7 @@ __device__ __noinline__ void op_kvwrite(const mdc_mega_params& p, int b) {
                                             (kv_row_base(L, b) + slot) * row_bytes);
       for (int i = tid; i < row_bytes / 16; i += kBlockThreads) dst[i] = src[i];
       // The row's LOGITS tasks read the page by TMA in this same launch: these stores are made visible to the async proxy
-      // before the task's notify releases them (the tile's copy warp fences on its side).
+      // before the task's notify releases them (op_logits fences on its side).
       if (tid < 32) fence_proxy_async_global();
       if (tid == 0) const_cast<int32_t*>(lp.seq_lens)[b] = slot + 1;
     }
@@ -273,6 +273,7 @@ __device__ __noinline__ int op_logits(const mdc_mega_params& p, const CUtensorMa
   const mdc_layer_params& L = p.layer;
   mdc_logits_params lp = L.logits;
   redirect_q(p, phase, &lp, nullptr);
+  if (L.kvw_glen) fence_proxy_async_global();   // the tile's TMA reads follow KVWRITE's ordinary stores to the page
   int n_list;   // (the same in all worker threads)
   if constexpr (THR) {
     const int64_t half = static_cast<int64_t>(L.B) * kThrBins;

@@ -339,8 +339,8 @@ struct RowExactSmem {
 
 constexpr int kSurvCap = 2048;   // scores of one chunk at or above the row's boundary bin (more: the row falls back)
 
-// Shared-memory scratch of the exact mode behind the chunk's histogram (all inside the idle raw ring).
-// (hs, kThrBins words, then this struct: checked against the ring's size where the tile is instantiated)
+// Shared-memory scratch of the exact mode with several ranks, in the raw ring, which is idle by then (its size is checked
+// where the tile is instantiated).
 struct RowExactScratch {
   uint32_t skey[kSurvCap];    // the chunk's survivors (keys in bins >= the boundary bin), in position order
   uint16_t spos[kSurvCap];    // ... and their positions inside the chunk
@@ -1283,7 +1283,6 @@ __device__ __forceinline__ int logits_tile(const mdc_logits_params& p, const CUt
       mbar_fence_init();
     }
     fence_proxy_async_smem();   // (the ring may have been the previous task's scratch)
-    if (!kAlone) fence_proxy_async_global();   // (a page may have been written by ordinary stores earlier in this launch)
     __syncwarp();
     int id = lane < n_pages ? bt[blk0 + lane] : -1;
     if (id >= p.num_pages) id = -1;
