@@ -24,8 +24,9 @@
 // issuing both spent 500 cycles per tile on waits and issue slots with the tensor core idle (2500
 // cycles per tile, of which the MMAs are 1540).
 //
-// Measured, 32 rows x 2048 selected slots: 64.9 -> 51.4 us; e4m3, 16 rows x 512 slots and the window: 58.3 us
-// on the mma.sync tile, 20.7 here.
+// Measured, 32 rows x 2048 selected slots: 65.4 us with one warp issuing both products -> 50.7 to 57.9 now, by the box (a box
+// gives the same time call after call, the boxes differ); e4m3, 16 rows x 512 slots and the window: 59.4 us on the mma.sync
+// tile, 17.2 here.
 //
 // Roles (448 threads): warps 0-3 softmax (thread = head: no cross-thread
 // reductions; reads S with tcgen05.ld, writes P with tcgen05.st, rescales O
