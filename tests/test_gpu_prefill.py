@@ -136,3 +136,35 @@ def test_chunks_on_new_tensors_on_another_stream():
         torch.cuda.synchronize()
         pf.check_status()
         assert all(torch.equal(r[k], want[k]) for r in got for k in want)
+
+
+def test_a_chunk_replays_from_a_cuda_graph():
+    """A chunk of two launches captured by its first call: replays follow the contents of the captured tensors."""
+    from mega_dsa_cp_b200.prefill import DsaPrefillChunk
+
+    S, K, tile, Tq = 4096, 512, 16, 48
+    caches, x = _chunk(S, Tq, K, seed=75)
+    first, new = tuple(t.clone() for t in x), tuple(t.flip(0).contiguous() for t in x)
+    wants = []
+    for y in (x, new):
+        pf = DsaPrefillChunk(tile, top_k=K, max_pages=S // 64, blocks_per_chunk=16)
+        pf.bind(*caches)
+        wants.append(_results(Tq, K))
+        pf.run(*y, **wants[-1])
+    torch.cuda.synchronize()
+    pf = DsaPrefillChunk(tile, top_k=K, max_pages=S // 64, blocks_per_chunk=16)
+    pf.bind(*caches)
+    got = _results(Tq, K)
+    got["out_lse"] = got["out_lse"].double()                # (one result copied inside the graph)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        pf.run(*x, **got)
+    for want, y in ((wants[0], x), (wants[1], new), (wants[0], x)):
+        for a, b in zip(x, y if y is new else first):
+            a.copy_(b)
+        for t in got.values():
+            t.zero_()      # (a row's ids behind its count are not written)
+        graph.replay()
+        torch.cuda.synchronize()
+        pf.check_status()
+        assert all(torch.equal(got[k], want[k].to(got[k].dtype)) for k in want)
