@@ -11,6 +11,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <mutex>
 
 #include "../../include/mdc.h"
 
@@ -309,20 +310,20 @@ extern "C" void mdc_set_last_cuda_error(int e);
 
 namespace mdc {
 // Raises a kernel's dynamic shared-memory limit to `bytes`.  The limit of a device only ever grows and is kept
-// here, so a launch does not go through the runtime for it every time.
+// here, so a launch does not go through the runtime for it every time.  (The runtime's call sets the limit, it does not
+// raise it: two threads' first launches take turns, or the smaller limit could be the one that stays.)
 constexpr int kMaxDevices = 64;
 template <auto Kernel>
 inline int allow_dynamic_smem(int bytes) {
   static std::atomic<int> limit[kMaxDevices];
+  static std::mutex raising;
   int dev = 0;
   MDC_CUDA_OK(cudaGetDevice(&dev));
   if (dev < kMaxDevices && limit[dev].load(std::memory_order_acquire) >= bytes) return MDC_OK;
+  std::lock_guard<std::mutex> lock(raising);
+  if (dev < kMaxDevices && limit[dev].load(std::memory_order_relaxed) >= bytes) return MDC_OK;
   MDC_CUDA_OK(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  if (dev < kMaxDevices) {
-    int have = limit[dev].load(std::memory_order_relaxed);
-    while (have < bytes && !limit[dev].compare_exchange_weak(have, bytes, std::memory_order_release)) {
-    }
-  }
+  if (dev < kMaxDevices) limit[dev].store(bytes, std::memory_order_release);
   return MDC_OK;
 }
 

@@ -531,3 +531,53 @@ def test_selection_with_ties_is_exact_on_own_logits(fmt, P, T, K, bpc, S, mode):
             n = int(rc[b, t])
             assert n == ei.numel() and torch.equal(ri[b, t, :n].cpu(), ei), (b, t)
             assert torch.equal(rv[b, t, :n].cpu().view(torch.int32), ev.view(torch.int32))
+
+
+FIRST_LAUNCHES = """
+import sys, threading
+sys.path.insert(0, %r)
+import torch
+from mega_dsa_cp_b200 import _native as N
+from mega_dsa_cp_b200.tiles.merge import run_merge_topk
+
+def call(L, K):
+    v = torch.randn(1, 1, L, K, device="cuda")
+    ids = torch.arange(L * K, dtype=torch.int32, device="cuda").view(1, 1, L, K)
+    out = [torch.zeros(1, 1, 64, device="cuda"), torch.zeros(1, 1, 64, dtype=torch.int32, device="cuda"), torch.zeros(1, 1, dtype=torch.int32, device="cuda")]
+    return v, ids, torch.full((1, 1, L), K, dtype=torch.int32, device="cuda"), *out, None
+
+calls = [call(1, 64 * i) for i in range(1, 33)] + [call(8, 2048)]
+N.host()
+torch.cuda.synchronize()
+together, failed = threading.Barrier(len(calls)), []
+
+def work(a):
+    together.wait()
+    run(a)
+
+def run(a):
+    try:
+        run_merge_topk(*a, stream=0, top_k=64)
+    except N.MdcError as e:
+        failed.append(str(e))
+
+threads = [threading.Thread(target=work, args=(a,)) for a in calls]
+for t in threads: t.start()
+for t in threads: t.join()
+for a in calls: run(a)
+torch.cuda.synchronize()
+assert all(int(a[5]) == 64 for a in calls)
+print("FAILED", len(failed))
+"""
+
+
+def test_first_launches_of_several_threads():
+    """A process's first launches of one kernel with different amounts of shared memory, from 33 threads at once: none may
+    leave the kernel's limit below what another one needs."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", FIRST_LAUNCHES % root], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.split()[-2:] == ["FAILED", "0"], r.stdout[-500:] + r.stderr[-1500:]
