@@ -387,7 +387,7 @@ __device__ __noinline__ void op_merge_l1a(const mdc_mega_params& p, int b, int g
   ls.stride = K;
   ls.c_stride = 1;
   const int64_t o = static_cast<int64_t>(b) * G + g;
-  merge_lists_auto<false>(ls, n, K, K, L.mid_v + o * K, L.mid_i + o * K, L.mid_c + o, nullptr, sm, smem + kMergeHdr,
+  merge_lists_auto<kLaunchLists>(ls, n, K, K, L.mid_v + o * K, L.mid_i + o * K, L.mid_c + o, nullptr, sm, smem + kMergeHdr,
                           kMegaTileSmem - kMergeHdr);
 }
 
@@ -423,7 +423,7 @@ __device__ __noinline__ void op_merge_l1(const mdc_mega_params& p, int b, unsign
   }
   const int64_t off = phase_offset(p, phase) + L.cand_off + (static_cast<int64_t>(b) * L.cp + L.rank) * cand_slice_bytes(L);
   unsigned char* slice = arena.local_ptr(off);
-  merge_lists_auto<false>(ls, C, K, K, reinterpret_cast<float*>(slice + kSliceV), reinterpret_cast<int32_t*>(slice + slice_i_off(K)),
+  merge_lists_auto<kLaunchLists>(ls, C, K, K, reinterpret_cast<float*>(slice + kSliceV), reinterpret_cast<int32_t*>(slice + slice_i_off(K)),
                           reinterpret_cast<int32_t*>(slice), nullptr, sm, smem + kMergeHdr, kMegaTileSmem - kMergeHdr);
   if (L.cp == 1) {
     // one rank: this list IS the selection; publish it and the gather list here (no MERGE_L2 task)
@@ -531,7 +531,7 @@ __device__ __noinline__ void op_merge_l2(const mdc_mega_params& p, int b, unsign
   // there, without a fence and two round trips to the copy in global memory.
   const int sid_bytes = (K * 4 + 15) & ~15;
   int32_t* sid = reinterpret_cast<int32_t*>(smem + kMegaTileSmem - sid_bytes);
-  const int n = merge_lists_auto<SYS>(ls, L.cp * cand_lists_per_rank(L), K, K, L.sel_v + static_cast<int64_t>(b) * K, sid, L.sel_c + b, nullptr, sm,
+  const int n = merge_lists_auto<SYS ? kPeerLists : kLaunchLists>(ls, L.cp * cand_lists_per_rank(L), K, K, L.sel_v + static_cast<int64_t>(b) * K, sid, L.sel_c + b, nullptr, sm,
                                      smem + kMergeHdr, kMegaTileSmem - kMergeHdr - sid_bytes);
   sync_workers();
   for (int i = threadIdx.x; i < n; i += kBlockThreads) sel_i[i] = sid[i];

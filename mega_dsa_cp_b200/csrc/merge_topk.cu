@@ -22,8 +22,8 @@ __device__ inline bool merge_row_by_hist(const mdc_merge_topk_params& p, int row
   uint32_t* hist = reinterpret_cast<uint32_t*>(ib) + n_pos;
   HistSelectSmem& hs = *reinterpret_cast<HistSelectSmem*>(hist + MDC_THR_BINS);
   for (int i = tid; i < MDC_THR_BINS / 4; i += kBlockThreads) reinterpret_cast<uint4*>(hist)[i] = make_uint4(0u, 0u, 0u, 0u);
-  merge_load_counts<false>(ls, p.L, p.maxK, sm);
-  merge_stage_lists<false>(ls, p.L, p.maxK, sm, vb, ib);
+  merge_load_counts<kInputLists>(ls, p.L, p.maxK, sm);
+  merge_stage_lists<kInputLists>(ls, p.L, p.maxK, sm, vb, ib);
   for (int i = tid; i < n_pos / 4; i += kBlockThreads) {
     const uint4 q = reinterpret_cast<const uint4*>(vb)[i];
     const uint32_t v[4] = {q.x, q.y, q.z, q.w};

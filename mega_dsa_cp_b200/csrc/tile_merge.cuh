@@ -41,18 +41,30 @@ struct MergeLists {
   int64_t stride, c_stride;
 };
 
-__device__ inline float ld_f32(const float* p, bool sys) { return sys ? ld_sys_f32(p) : __ldg(p); }
+// Who wrote the lists: an earlier launch (the read-only path may be used: 8 queries x 4 lists of 2048 8.35 us, 8.6 with ordinary
+// loads), other blocks during this one, or peer GPUs (loads must bypass the L1).
+enum ListOrigin { kInputLists, kLaunchLists, kPeerLists };
+template <ListOrigin W>
+__device__ inline float ld_f32(const float* p) {
+  if (W == kPeerLists) return ld_sys_f32(p);
+  return W == kInputLists ? __ldg(p) : *p;
+}
+template <ListOrigin W>
+__device__ inline uint4 ld_u4(const void* p) {
+  const uint4* q = static_cast<const uint4*>(p);
+  if (W == kPeerLists) return ld_sys_u4(q);
+  return W == kInputLists ? __ldg(q) : *q;
+}
 
-// SYS: the lists were written by peer GPUs (loads must bypass the L1).
 // Called by the 256 worker threads.  out_v / out_i / out_c point at this row's output.
-template <bool SYS>
+template <ListOrigin W>
 __device__ inline int merge_lists_tile(const MergeLists& ls, int L, int maxK, int top_k, float* out_v, int32_t* out_i,
                                        int32_t* out_c, int32_t* dbg, MergeSmem& sm) {
   const int tid = threadIdx.x;
   sync_workers();
   for (int l = tid; l < L; l += kBlockThreads) {
     const int32_t* cp = ls.c + l * ls.c_stride;
-    int c = SYS ? __float_as_int(ld_sys_f32(reinterpret_cast<const float*>(cp))) : *cp;
+    int c = W == kPeerLists ? __float_as_int(ld_sys_f32(reinterpret_cast<const float*>(cp))) : *cp;
     sm.cnt[l] = max(0, min(c, maxK));
   }
   sync_workers();
@@ -60,8 +72,8 @@ __device__ inline int merge_lists_tile(const MergeLists& ls, int L, int maxK, in
     const int l = pos / maxK, j = pos - l * maxK;
     valid = j < sm.cnt[l];
     if (!valid) return 0ull;
-    const uint32_t hi = sortable_u32(ld_f32(ls.v + l * ls.stride + j, SYS));
-    const uint32_t lo = ~static_cast<uint32_t>(__float_as_int(ld_f32(reinterpret_cast<const float*>(ls.i + l * ls.stride + j), SYS)));
+    const uint32_t hi = sortable_u32(ld_f32<W>(ls.v + l * ls.stride + j));
+    const uint32_t lo = ~static_cast<uint32_t>(__float_as_int(ld_f32<W>(reinterpret_cast<const float*>(ls.i + l * ls.stride + j))));
     return (static_cast<unsigned long long>(hi) << 32) | lo;
   };
   const int n_pos = L * maxK;
@@ -69,8 +81,8 @@ __device__ inline int merge_lists_tile(const MergeLists& ls, int L, int maxK, in
   int n = block_emit_selected<unsigned long long>(src, n_pos, th, sm.sel, [&](int pos, int slot) {
     if (slot < top_k) {
       const int l = pos / maxK, j = pos - l * maxK;
-      out_v[slot] = ld_f32(ls.v + l * ls.stride + j, SYS);
-      out_i[slot] = __float_as_int(ld_f32(reinterpret_cast<const float*>(ls.i + l * ls.stride + j), SYS));
+      out_v[slot] = ld_f32<W>(ls.v + l * ls.stride + j);
+      out_i[slot] = __float_as_int(ld_f32<W>(reinterpret_cast<const float*>(ls.i + l * ls.stride + j)));
     }
   });
   if (tid == 0) {
@@ -83,7 +95,7 @@ __device__ inline int merge_lists_tile(const MergeLists& ls, int L, int maxK, in
 // Register-resident path of merge_lists_tile for L * maxK <= 256 * E: one read
 // of the lists, a u32 select on the logits, and -- only when equal logits
 // straddle the boundary -- a second u32 select on ~id among the tied entries.
-template <int E, bool SYS>
+template <int E, ListOrigin W>
 __device__ inline int merge_lists_regs(const MergeLists& ls, int L, int maxK, int top_k, float* out_v, int32_t* out_i,
                                        int32_t* out_c, int32_t* dbg, MergeSmem& sm) {
   const int tid = threadIdx.x;
@@ -91,7 +103,7 @@ __device__ inline int merge_lists_regs(const MergeLists& ls, int L, int maxK, in
   sync_workers();
   for (int l = tid; l < L; l += kBlockThreads) {
     const int32_t* cp = ls.c + l * ls.c_stride;
-    int c = SYS ? __float_as_int(ld_sys_f32(reinterpret_cast<const float*>(cp))) : *cp;
+    int c = W == kPeerLists ? __float_as_int(ld_sys_f32(reinterpret_cast<const float*>(cp))) : *cp;
     sm.cnt[l] = max(0, min(c, maxK));
   }
   sync_workers();
@@ -102,7 +114,7 @@ __device__ inline int merge_lists_regs(const MergeLists& ls, int L, int maxK, in
     key[it] = 0u;
     if (pos < n_pos) {
       const int l = pos / maxK, j = pos - l * maxK;
-      if (j < sm.cnt[l]) key[it] = max(sortable_u32(ld_f32(ls.v + l * ls.stride + j, SYS)), 1u);
+      if (j < sm.cnt[l]) key[it] = max(sortable_u32(ld_f32<W>(ls.v + l * ls.stride + j)), 1u);
     }
   }
   const Threshold<uint32_t> th = block_select_regs<E>(key, top_k, sm.rsel);
@@ -126,7 +138,7 @@ __device__ inline int merge_lists_regs(const MergeLists& ls, int L, int maxK, in
         uint32_t k2 = 0u;
         if ((tie_m >> it) & 1ull) {
           const int l = pos / maxK, j = pos - l * maxK;
-          k2 = ~static_cast<uint32_t>(__float_as_int(ld_f32(reinterpret_cast<const float*>(ls.i + l * ls.stride + j), SYS)));
+          k2 = ~static_cast<uint32_t>(__float_as_int(ld_f32<W>(reinterpret_cast<const float*>(ls.i + l * ls.stride + j))));
           k2 = max(k2, 1u);
         }
         key[it] = k2;
@@ -157,8 +169,8 @@ __device__ inline int merge_lists_regs(const MergeLists& ls, int L, int maxK, in
     if (slot[it] >= 0 && slot[it] < top_k) {
       const int pos = it * kBlockThreads + tid;
       const int l = pos / maxK, j = pos - l * maxK;
-      out_v[slot[it]] = ld_f32(ls.v + l * ls.stride + j, SYS);
-      out_i[slot[it]] = __float_as_int(ld_f32(reinterpret_cast<const float*>(ls.i + l * ls.stride + j), SYS));
+      out_v[slot[it]] = ld_f32<W>(ls.v + l * ls.stride + j);
+      out_i[slot[it]] = __float_as_int(ld_f32<W>(reinterpret_cast<const float*>(ls.i + l * ls.stride + j)));
     }
   }
   if (tid == 0) {
@@ -172,19 +184,19 @@ __device__ inline int merge_lists_regs(const MergeLists& ls, int L, int maxK, in
 // of the logit (0 = empty position), ib[pos] = id.  The loads carry no branch
 // (invalid positions read element 0 of their list and are masked afterwards),
 // so a thread's loads of one batch are all in flight together.
-template <bool SYS>
+template <ListOrigin W>
 __device__ inline void merge_load_counts(const MergeLists& ls, int L, int maxK, MergeSmem& sm) {
   sync_workers();
   for (int l = threadIdx.x; l < L; l += kBlockThreads) {
     const int32_t* cp = ls.c + l * ls.c_stride;
-    int c = SYS ? __float_as_int(ld_sys_f32(reinterpret_cast<const float*>(cp))) : *cp;
+    int c = W == kPeerLists ? __float_as_int(ld_sys_f32(reinterpret_cast<const float*>(cp))) : *cp;
     sm.cnt[l] = max(0, min(c, maxK));
   }
   sync_workers();
 }
 
 // counts must have been loaded (merge_load_counts)
-template <bool SYS>
+template <ListOrigin W>
 __device__ inline void merge_stage_lists(const MergeLists& ls, int L, int maxK, MergeSmem& sm, uint32_t* vb, int32_t* ib) {
   const int tid = threadIdx.x;
   const int n_pos = L * maxK;
@@ -195,8 +207,7 @@ __device__ inline void merge_stage_lists(const MergeLists& ls, int L, int maxK, 
     constexpr int U = 8;
     const int n_vec = n_pos >> 2, k4 = maxK >> 2;
     for (int q0 = tid; q0 < n_vec; q0 += U * kBlockThreads) {
-      float4 v[U];
-      int4 f[U];
+      uint4 v[U], f[U];
       int cnt[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -204,27 +215,20 @@ __device__ inline void merge_stage_lists(const MergeLists& ls, int L, int maxK, 
         const int l = qi / k4, j = (qi - l * k4) << 2;
         cnt[u] = sm.cnt[l] - j;  // valid positions of this quad: those below cnt
         const int64_t off = l * ls.stride + j;
-        if (SYS) {  // lists written by peer GPUs: system-scope loads that bypass the L1
-          const uint4 a = ld_sys_u4(reinterpret_cast<const uint4*>(ls.v + off));
-          const uint4 b = ld_sys_u4(reinterpret_cast<const uint4*>(ls.i + off));
-          v[u] = make_float4(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z), __uint_as_float(a.w));
-          f[u] = make_int4(static_cast<int>(b.x), static_cast<int>(b.y), static_cast<int>(b.z), static_cast<int>(b.w));
-        } else {
-          v[u] = __ldg(reinterpret_cast<const float4*>(ls.v + off));
-          f[u] = __ldg(reinterpret_cast<const int4*>(ls.i + off));
-        }
+        v[u] = ld_u4<W>(ls.v + off);
+        f[u] = ld_u4<W>(ls.i + off);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int qi = q0 + u * kBlockThreads;
         if (qi < n_vec) {
           uint4 kv;
-          kv.x = cnt[u] > 0 ? max(sortable_u32(v[u].x), 1u) : 0u;
-          kv.y = cnt[u] > 1 ? max(sortable_u32(v[u].y), 1u) : 0u;
-          kv.z = cnt[u] > 2 ? max(sortable_u32(v[u].z), 1u) : 0u;
-          kv.w = cnt[u] > 3 ? max(sortable_u32(v[u].w), 1u) : 0u;
+          kv.x = cnt[u] > 0 ? max(sortable_u32(__uint_as_float(v[u].x)), 1u) : 0u;
+          kv.y = cnt[u] > 1 ? max(sortable_u32(__uint_as_float(v[u].y)), 1u) : 0u;
+          kv.z = cnt[u] > 2 ? max(sortable_u32(__uint_as_float(v[u].z)), 1u) : 0u;
+          kv.w = cnt[u] > 3 ? max(sortable_u32(__uint_as_float(v[u].w)), 1u) : 0u;
           reinterpret_cast<uint4*>(vb)[qi] = kv;
-          if (ib) reinterpret_cast<int4*>(ib)[qi] = f[u];
+          if (ib) reinterpret_cast<uint4*>(ib)[qi] = f[u];
         }
       }
     }
@@ -242,8 +246,8 @@ __device__ inline void merge_stage_lists(const MergeLists& ls, int L, int maxK, 
       const bool in = pos0 + u * kBlockThreads < n_pos;
       ok[u] = in && j < sm.cnt[in ? l : 0];
       const int64_t off = ok[u] ? l * ls.stride + j : 0;
-      v[u] = ld_f32(ls.v + off, SYS);
-      f[u] = ld_f32(reinterpret_cast<const float*>(ls.i) + off, SYS);
+      v[u] = ld_f32<W>(ls.v + off);
+      f[u] = ld_f32<W>(reinterpret_cast<const float*>(ls.i) + off);
       l += dl;
       j += dj;
       if (j >= maxK) {
@@ -268,7 +272,7 @@ __device__ inline void merge_stage_lists(const MergeLists& ls, int L, int maxK, 
 // entries are staged, list after list, so the search and the emit run over sum(cnt) positions instead
 // of L * maxK.  The staged order is the padded order without its holes: same output.  Returns the
 // staged length, padded with empty positions to a multiple of four.
-template <bool SYS>
+template <ListOrigin W>
 __device__ inline int merge_stage_compact(const MergeLists& ls, int L, MergeSmem& sm, uint32_t* vb, int32_t* ib,
                                            bool max_quads_ok = false) {
   const int tid = threadIdx.x, lane = tid & 31;
@@ -331,13 +335,8 @@ __device__ inline int merge_stage_compact(const MergeLists& ls, int L, MergeSmem
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int64_t at = li[u] >= 0 ? li[u] * ls.stride + j[u] : 0;
-        if (SYS) {
-          a[u] = ld_sys_u4(reinterpret_cast<const uint4*>(ls.v + at));
-          bq[u] = ld_sys_u4(reinterpret_cast<const uint4*>(ls.i + at));
-        } else {
-          a[u] = __ldg(reinterpret_cast<const uint4*>(ls.v + at));
-          bq[u] = __ldg(reinterpret_cast<const uint4*>(ls.i + at));
-        }
+        a[u] = ld_u4<W>(ls.v + at);
+        bq[u] = ld_u4<W>(ls.i + at);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -382,8 +381,8 @@ __device__ inline int merge_stage_compact(const MergeLists& ls, int L, MergeSmem
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t at = src[u] >= 0 ? src[u] : 0;   // (an empty position reads element 0 and is masked below)
-      v[u] = ld_f32(ls.v + at, SYS);
-      f[u] = ld_f32(reinterpret_cast<const float*>(ls.i) + at, SYS);
+      v[u] = ld_f32<W>(ls.v + at);
+      f[u] = ld_f32<W>(reinterpret_cast<const float*>(ls.i) + at);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -580,14 +579,14 @@ __device__ inline int merge_prefilter(const uint32_t* vb, const int32_t* ib, int
 // Picks the fastest path the row size allows: staged in shared memory (when
 // `stage` offers 8 bytes per position) with register or shared-memory keys,
 // else register keys read from global memory, else re-reading global memory per pass.
-template <bool SYS>
+template <ListOrigin W>
 __device__ inline int merge_lists_auto(const MergeLists& ls, int L, int maxK, int top_k, float* out_v, int32_t* out_i,
                                        int32_t* out_c, int32_t* dbg, MergeSmem& sm, unsigned char* stage = nullptr,
                                        int stage_bytes = 0) {
   int n_pos = L * maxK;
   int n_valid = -1;
   if (stage && maxK >= 1) {
-    merge_load_counts<SYS>(ls, L, maxK, sm);
+    merge_load_counts<W>(ls, L, maxK, sm);
     n_valid = 0;
     for (int l = 0; l < L; ++l) n_valid += sm.cnt[l];
   }
@@ -597,8 +596,8 @@ __device__ inline int merge_lists_auto(const MergeLists& ls, int L, int maxK, in
   if (stage && maxK >= 1 && (compact || n_pos * 8 <= stage_bytes)) {
     uint32_t* vb = reinterpret_cast<uint32_t*>(stage);
     int32_t* ib = reinterpret_cast<int32_t*>(stage) + (compact ? n_cap : n_pos);
-    if (compact) n_pos = merge_stage_compact<SYS>(ls, L, sm, vb, ib, (maxK & 3) == 0);
-    else merge_stage_lists<SYS>(ls, L, maxK, sm, vb, ib);
+    if (compact) n_pos = merge_stage_compact<W>(ls, L, sm, vb, ib, (maxK & 3) == 0);
+    else merge_stage_lists<W>(ls, L, maxK, sm, vb, ib);
     {
       // Nothing to select when the lists hold no more than top_k entries between them (one rank's
       // list passing through the cross-rank merge, short contexts): every valid position is
@@ -645,15 +644,15 @@ __device__ inline int merge_lists_auto(const MergeLists& ls, int L, int maxK, in
   if (stage && n_pos * 4 <= stage_bytes && maxK >= 1) {
     // too long for keys + ids: stage the keys only, fetch the few ids that are needed from global memory
     uint32_t* vb = reinterpret_cast<uint32_t*>(stage);
-    merge_stage_lists<SYS>(ls, L, maxK, sm, vb, nullptr);
+    merge_stage_lists<W>(ls, L, maxK, sm, vb, nullptr);
     return merge_staged_bits(n_pos, top_k, out_v, out_i, out_c, dbg, sm, vb, [&](int pos) {
       const int l = pos / maxK, j = pos - l * maxK;
-      return __float_as_int(ld_f32(reinterpret_cast<const float*>(ls.i + l * ls.stride + j), SYS));
+      return __float_as_int(ld_f32<W>(reinterpret_cast<const float*>(ls.i + l * ls.stride + j)));
     });
   }
   if (n_pos <= kBlockThreads * kMergeRegE)
-    return merge_lists_regs<kMergeRegE, SYS>(ls, L, maxK, top_k, out_v, out_i, out_c, dbg, sm);
-  return merge_lists_tile<SYS>(ls, L, maxK, top_k, out_v, out_i, out_c, dbg, sm);
+    return merge_lists_regs<kMergeRegE, W>(ls, L, maxK, top_k, out_v, out_i, out_c, dbg, sm);
+  return merge_lists_tile<W>(ls, L, maxK, top_k, out_v, out_i, out_c, dbg, sm);
 }
 
 // stage = optional dynamic shared memory of stage_bytes for the shared-memory path
@@ -666,7 +665,7 @@ __device__ inline void merge_topk_tile(const mdc_merge_topk_params& p, int row, 
   ls.c = p.cand_c + static_cast<int64_t>(row) * p.L;
   ls.stride = p.maxK;
   ls.c_stride = 1;
-  merge_lists_auto<false>(ls, p.L, p.maxK, p.top_k, p.out_v + static_cast<int64_t>(row) * p.top_k,
+  merge_lists_auto<kInputLists>(ls, p.L, p.maxK, p.top_k, p.out_v + static_cast<int64_t>(row) * p.top_k,
                           p.out_i + static_cast<int64_t>(row) * p.top_k, p.out_c + row, p.dbg, sm, stage, stage_bytes);
 }
 

@@ -127,7 +127,7 @@ __device__ inline void mla_load_tile(const mdc_sparse_mla_params& p, int r, int 
       const unsigned char* src = mla_slot_ptr<DQK, 1>(p, r, slot0 + s, k_valid, win_valid);
       if (ch == 0) sValid[s] = src != nullptr;
       uint4 raw = make_uint4(0, 0, 0, 0);
-      if (src) raw = __ldg(reinterpret_cast<const uint4*>(src + ch * 16));
+      if (src) raw = *reinterpret_cast<const uint4*>(src + ch * 16);   // (not the read-only path: KVWRITE may have written the row in this launch)
       uint4 lo, hi;
       e4m3x4_to_bf16(raw.x, lo.x, lo.y);
       e4m3x4_to_bf16(raw.y, lo.z, lo.w);
