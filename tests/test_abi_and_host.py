@@ -209,20 +209,6 @@ def test_layers_with_a_row_threshold_stay_within_its_chunks():
         assert plain.bpc == 32000 // page
 
 
-def test_only_rows_that_settle_themselves_are_cut_into_one_wave_of_chunks():
-    """One sequence of 131072 tokens: as many chunks as blocks where the chunk tasks settle the row between them; the
-    chunks that were asked for where a merge task has to read their lists."""
-    from mega_dsa_cp_b200.layer import DsaDecodeLayer
-
-    make = lambda **kw: DsaDecodeLayer(1, max_pages=2048, blocks_per_chunk=128, n_ctas=148, device="cpu", **kw)
-    for kw in (dict(top_k=2048), dict(top_k=2048, row_exact=True)):
-        layer = make(**kw)
-        assert (layer.row_exact, layer.bpc, layer.n_chunks) == (4, 14, 147), kw
-    for kw in (dict(top_k=2046), dict(top_k=2048, row_exact=False), dict(top_k=2048, row_exact="local"), dict(top_k=2048, row_threshold=False)):
-        layer = make(**kw)
-        assert (layer.row_exact, layer.bpc, layer.n_chunks) == (0, 128, 16), kw
-
-
 def test_indexer_check_refuses_misaligned_queries():
     """bf16 query rows are read in 16-byte pieces, FP4 rows in 4-byte ones (8 is what has been asked for)."""
     from mega_dsa_cp_b200 import _native as N
