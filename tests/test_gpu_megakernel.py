@@ -603,7 +603,7 @@ def test_merge_task_passes_on_what_the_chunk_tasks_published():
     g = torch.Generator().manual_seed(82)
     seq = torch.tensor([S, S, S - 70, K // 3], dtype=torch.int32)
     layer = DsaDecodeLayer(B, top_k=K, max_pages=S // P, blocks_per_chunk=32, kv_seq_stride=S, out_dtype=torch.float32, n_ctas=64, row_exact=False)
-    assert layer.n_chunks == 4 and layer.n_dag_events == layer.events.num_events
+    assert layer.n_chunks == 16 and layer.n_dag_events == layer.events.num_events
     layer.row_exact = 1
     layer.events = alloc_event_buffer(layer.n_dag_events + 2 * B, device=layer.device)
     layer.arena = alloc_arena(arena_regions(B, 1, K, H, layer.attn_splits, thr_chunks=layer.n_chunks), layer.phases, device=layer.device)
