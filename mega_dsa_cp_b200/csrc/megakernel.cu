@@ -912,6 +912,10 @@ static int layer_check(const mdc_mega_params& p) {
   if (pieces & 15) return MDC_ERR_BAD_ALIGN;
   if (L.l1_groups > 1 && (!L.mid_v || !L.mid_i || !L.mid_c)) return MDC_ERR_NULL;
   if (L.l1_groups < 0 || L.l1_groups > L.n_chunks) return MDC_ERR_BAD_SHAPE;
+  {  // a merge holds 256 lists: the chunks, or their groups and the chunks of a group
+    const int groups = L.l1_groups > 1 ? L.l1_groups : 1, first = ceil_div(L.n_chunks, groups), last = groups > 1 ? groups : L.n_chunks;
+    if (!(L.cand_direct && L.cp > 1) && (first > kMergeMaxLists || last > kMergeMaxLists)) return MDC_ERR_TOO_LARGE;
+  }
   if (L.cand_direct && L.cp > 1 && (L.l1_groups > 1 || L.cp * L.n_chunks > 256)) return MDC_ERR_BAD_SHAPE;  // the merge takes 256 lists
   if (L.cand_direct && L.cp > 1 && L.top_k % 4 != 0) return MDC_ERR_BAD_ALIGN;   // the ids start on a 16-byte boundary of the slice
   if (L.thr_exact) {

@@ -209,6 +209,33 @@ def test_layers_with_a_row_threshold_stay_within_its_chunks():
         assert plain.bpc == 32000 // page
 
 
+def test_megakernel_check_refuses_more_lists_than_a_merge_holds():
+    """A merge keeps the counts of 256 lists: chunks merged at once, groups of them, chunks of a group."""
+    from mega_dsa_cp_b200 import _native as N
+
+    for chunks, groups, want in ((256, 1, 0), (257, 1, -6), (1024, 256, 0), (1028, 257, -6), (513, 2, -6), (512, 2, 0)):
+        p = _valid_mega_params(N)
+        L = p.layer
+        L.n_chunks = L.logits.n_chunks = chunks
+        L.l1_groups, L.mid_v, L.mid_i, L.mid_c = groups, 1 << 20, 1 << 20, 1 << 20
+        assert N.lib().mdc_megakernel_check(C.byref(p)) == want, (chunks, groups)
+
+
+def test_layers_of_many_chunks_take_merges_that_hold_them():
+    """A row's chunk tasks wait for each other under the row threshold, so all of them must run at once; more chunks go
+    without it, in groups that one merge can read."""
+    from mega_dsa_cp_b200.layer import DsaDecodeLayer, l1_groups_for
+
+    make = lambda **kw: DsaDecodeLayer(1, top_k=64, blocks_per_chunk=1, device="cpu", **kw)
+    layer = make(max_pages=148, n_ctas=148)
+    assert layer.row_threshold and layer.row_exact == 4 and layer.n_chunks == 148 and layer.l1_groups == 1
+    for pages, ctas in ((149, 148), (300, 148), (300, 400), (2048, 148)):
+        layer = make(max_pages=pages, n_ctas=ctas)
+        assert not layer.row_threshold and layer.thr_hist is None and not layer.row_exact and layer.n_chunks == pages
+        assert 1 < layer.l1_groups <= 256 and -(-layer.n_chunks // layer.l1_groups) <= 256
+    assert [l1_groups_for(n) for n in (8, 9, 16, 20, 1024)] == [1, 3, 4, 5, 256]
+
+
 def test_indexer_check_refuses_misaligned_queries():
     """bf16 query rows are read in 16-byte pieces, FP4 rows in 4-byte ones (8 is what has been asked for)."""
     from mega_dsa_cp_b200 import _native as N

@@ -626,3 +626,36 @@ def test_merge_task_passes_on_what_the_chunk_tasks_published():
             assert n == ei.numel() and torch.equal(layer.sel_i[b, :n].cpu(), ei), b
             assert torch.equal(layer.sel_v[b, :n].cpu().view(torch.int32), ev.view(torch.int32)), b
             assert torch.equal(layer.pt_local[b, :n].cpu(), ei + b * S) and int(layer.k_valid[b]) == 128 + n
+
+
+@pytest.mark.parametrize("B,pages,K,n_ctas", [(2, 300, 512, 148), (1, 1030, 2048, 148), (3, 40, 64, 31)])
+def test_rows_of_more_chunks_than_blocks(B, pages, K, n_ctas):
+    """One page per chunk (blocks_per_chunk = 1), more chunks than blocks or than one merge holds: the chunks' exact lists
+    and two levels of merges, against the top-k of the kernel's own logits."""
+    from dsa_inputs import indexer_case
+    from mega_dsa_cp_b200.layer import DsaDecodeLayer, LayerInputs
+    from mega_dsa_cp_b200.tiles.logits import run_fp4_paged_mqa_logits
+    from oracle import dsa_oracle as orc
+
+    P, H, DQK = 64, 128, 576
+    S = pages * P
+    case = indexer_case(B, S, P, "nvfp4", seed=91)
+    g = torch.Generator().manual_seed(92)
+    seq = torch.tensor([S, S - 1000, 77][:B], dtype=torch.int32)
+    layer = DsaDecodeLayer(B, top_k=K, max_pages=pages, blocks_per_chunk=1, kv_seq_stride=S, out_dtype=torch.float32, n_ctas=n_ctas)
+    assert layer.n_chunks == pages and layer.l1_groups > 1
+    d = lambda t: t.to(DEV)
+    layer.bind(LayerInputs(d(case["fused"]), d(case["bt"]), d(seq), d(case["q"]), d(case["w"]),
+                           d((torch.randn(B, 1, H, DQK, generator=g) * 0.5).bfloat16()),
+                           d((torch.randn(B * S, 1, DQK, generator=g) * 0.5).bfloat16())))
+    logits = torch.zeros(B, S, device=DEV)
+    run_fp4_paged_mqa_logits(d(case["fused"]), d(case["q"]), None, d(case["w"]), d(case["bt"]), logits, 16, fmt="nvfp4", page_tokens=P)
+    for _ in range(2):
+        layer.step()
+        torch.cuda.synchronize()
+        layer.check_status()
+        for b in range(B):
+            ev, ei = orc.local_topk_ref(logits[b].cpu(), 0, S, int(seq[b]), K, 1, 0)
+            n = int(layer.sel_c[b])
+            assert n == ei.numel() and torch.equal(layer.sel_i[b, :n].cpu(), ei), b
+            assert torch.equal(layer.sel_v[b, :n].cpu().view(torch.int32), ev.view(torch.int32)), b
