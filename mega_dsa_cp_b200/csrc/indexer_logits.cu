@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(kLogitsThreads, 1) logits_kernel(const __grid_
   let_successor_start();
   // the UMMA operand block wants a 1024-byte aligned base
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  logits_tile<FMT, PAGE, T, kLogitsDecodeGroups, kLogitsGateGroups, kLogitsIssueWarps>(p, &pages, blockIdx.y, blockIdx.x, smem);
+  logits_tile<FMT, PAGE, T, true>(p, &pages, blockIdx.y, blockIdx.x, smem);
 }
 
 // Row mode: the blocks of one request form a cluster and select across their chunks.
@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kLogitsThreads, 1) logits_row_kernel(const __g
   extern __shared__ unsigned char smem_raw[];
   wait_for_predecessor();
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  logits_tile<FMT, PAGE, T, kLogitsDecodeGroups, kLogitsGateGroups, kLogitsIssueWarps, true>(p, &pages, blockIdx.y, blockIdx.x, smem);
+  logits_tile<FMT, PAGE, T, true, true>(p, &pages, blockIdx.y, blockIdx.x, smem);
 }
 
 template <int FMT, int PAGE, int T>

@@ -4,8 +4,8 @@
 // Cross-rank payload travels by direct stores / bulk copies into the peers'
 // symmetric arena, followed by a system-scope release notify.
 //
-// Block shape: 15 warps.  Warps 0..7 are the workers every tile is written
-// for; the indexer tile additionally uses warps 8..14 (gate, issue, copy).
+// Block shape: 16 warps, which leave a thread 128 registers.  Warps 0..7 are the workers every tile is written
+// for; the indexer, attention and LSE-merge tiles use the others too.
 // Blocks wait on each other, so the grid must be co-resident (<= one block per
 // SM; the launcher checks it).  Every wait has a time budget; a block that
 // runs out records the event in the status block, which all blocks check at
@@ -24,11 +24,7 @@
 
 namespace mdc {
 
-// Gate groups and issue warps of the indexer tile inside the persistent kernel.  A second gate group would leave every thread
-// 96 registers, and the other tasks lose more than the indexer gains (layer-step of 8 sequences 107.7 us; 114.4 with
-// two groups).
-constexpr int kMegaGate = 1, kMegaIssue = 1;
-constexpr int kMegaThreads = logits_threads(2, kMegaGate, kMegaIssue);
+constexpr int kMegaThreads = kLogitsThreads;
 static_assert(kMegaThreads >= kMuThreads, "the block must hold the attention tile's warps (its roles go by warp index; extra warps only join the barriers)");
 constexpr int kStagedWords = 128;  // queue rows up to this length are staged in shared memory
 constexpr int kMegaTileSmem = MlaUmmaSmem<576>::kTotal > MlaSmem<576>::kTotal ? MlaUmmaSmem<576>::kTotal : MlaSmem<576>::kTotal;  // the largest tile
@@ -51,7 +47,7 @@ struct MegaShared {
   int32_t row[kStagedWords];
   int32_t fail;
   int32_t next;   // dynamic scheduling: index of the task this block pulled
-  unsigned long long phase;
+  unsigned long long phase, tr0, tr1;   // (tr0, tr1: the task's times for the trace)
 };
 
 __device__ inline int64_t phase_offset(const mdc_mega_params& p, unsigned long long phase) {
@@ -266,9 +262,9 @@ __device__ inline void redirect_q(const mdc_mega_params& p, unsigned long long p
 }
 
 // Returns the length of the chunk's candidate list (to the worker threads alike), -1 when the row has been published.
-// THR: with the row threshold (a function of its own: what the tile does then is known when it is compiled).
+// THR: with the row threshold (what the tile does then is known when it is compiled).
 template <int FMT, int PAGE, bool THR>
-__device__ __noinline__ int op_logits(const mdc_mega_params& p, const CUtensorMap* pages, int b, int chunk, unsigned long long phase,
+__device__ __forceinline__ int op_logits(const mdc_mega_params& p, const CUtensorMap* pages, int b, int chunk, unsigned long long phase,
                                        unsigned char* smem) {
   const mdc_layer_params& L = p.layer;
   mdc_logits_params lp = L.logits;
@@ -327,9 +323,9 @@ __device__ __noinline__ int op_logits(const mdc_mega_params& p, const CUtensorMa
       }
       rt.x = &x;
     }
-    n_list = logits_tile<FMT, PAGE, 1, 2, kMegaGate, kMegaIssue>(lp, pages, b, chunk, smem, &rt);
+    n_list = logits_tile<FMT, PAGE, 1, false, false, true>(lp, pages, b, chunk, smem, &rt);
   } else {
-    n_list = logits_tile<FMT, PAGE, 1, 2, kMegaGate, kMegaIssue>(lp, pages, b, chunk, smem);
+    n_list = logits_tile<FMT, PAGE, 1, false>(lp, pages, b, chunk, smem);
   }
   if (L.cand_direct && L.cp > 1 && threadIdx.x < kBlockThreads) {
     // The chunk's list goes to every rank's candidate region (slot rank * n_chunks + chunk of the
@@ -371,6 +367,15 @@ __device__ __noinline__ int op_logits(const mdc_mega_params& p, const CUtensorMa
     sync_workers();
   }
   return n_list;
+}
+
+// The operations of the default layer (NVFP4 pages of 64 tokens, row threshold, bf16 attention over 576 dims, LSE merge) stand
+// in the kernel's body: a call keeps 32 registers from a function, which has to save them.  The other forms are functions, to
+// keep the body short (step of 8 x 131072 with all of them functions 83.3 us, with these three inside 79.1).
+template <int FMT, int PAGE, bool THR>
+__device__ __noinline__ int op_logits_call(const mdc_mega_params& p, const CUtensorMap* pages, int b, int chunk, unsigned long long phase,
+                                           unsigned char* smem) {
+  return op_logits<FMT, PAGE, THR>(p, pages, b, chunk, phase, smem);
 }
 
 // first level of a two-level local merge: the chunk lists of group g of sequence b -> one list
@@ -544,8 +549,7 @@ __device__ __noinline__ void op_merge_l2(const mdc_mega_params& p, int b, unsign
 // (bf16) and its log2-LSE go straight into the owner's inbox.  With bf16 operands and heads in
 // blocks of 128 a task is 128 heads x 128 output columns on the tcgen05 tile (task index =
 // 4 * head block + column block, all threads take part); otherwise 64 heads x 256 columns on
-// the mma.sync tile (task index = 2 * head block + column half, worker threads only).  Each tile is a function of its own:
-// together in one they spill.
+// the mma.sync tile (task index = 2 * head block + column half, worker threads only).
 struct AttnTarget {
   unsigned char* slot;   // the partial's (H, 512) block in the owner's inbox
   float* lse_row;
@@ -573,11 +577,16 @@ __device__ inline mdc_sparse_mla_params attn_params(const mdc_mega_params& p, in
   return mp;
 }
 template <int DQK>
-__device__ __noinline__ void op_attn_umma(const mdc_mega_params& p, int b, int hbv, int split, unsigned long long phase,
+__device__ __forceinline__ void op_attn_umma(const mdc_mega_params& p, int b, int hbv, int split, unsigned long long phase,
                                           unsigned char* smem) {
   const AttnTarget t = attn_target(p, b, split, phase);
   const mdc_sparse_mla_params mp = attn_params(p, b, phase);
   mla_umma_tile<DQK>(mp, b, hbv >> 2, hbv & 3, t.split, t.ns, smem, t.slot, t.lse_row, true);
+}
+template <int DQK>
+__device__ __noinline__ void op_attn_umma_call(const mdc_mega_params& p, int b, int hbv, int split, unsigned long long phase,
+                                               unsigned char* smem) {
+  op_attn_umma<DQK>(p, b, hbv, split, phase, smem);
 }
 template <int DQK, int KVDT>
 __device__ __noinline__ void op_attn_mma(const mdc_mega_params& p, int b, int hbv, int split, unsigned long long phase,
@@ -595,7 +604,7 @@ __device__ inline void op_attn(const mdc_mega_params& p, int b, int hbv, int spl
   const bool bf16 = L.mla.kv_dtype == MDC_DT_BF16, wide = L.mla.d_qk == 576;
   if (bf16 && L.H % kMuHeads == 0) {
     if (wide) op_attn_umma<576>(p, b, hbv, split, phase, smem);
-    else op_attn_umma<512>(p, b, hbv, split, phase, smem);
+    else op_attn_umma_call<512>(p, b, hbv, split, phase, smem);
     return;
   }
   if (threadIdx.x >= kBlockThreads) return;
@@ -608,7 +617,7 @@ __device__ inline void op_attn(const mdc_mega_params& p, int b, int hbv, int spl
 // owner of sequence b: cp inbox slices -> merged output
 // (task = head group hq of n_groups: the merge of one sequence is spread over several blocks)
 template <bool SYS>
-__device__ __noinline__ void op_lse_merge(const mdc_mega_params& p, int b, int hq, int n_groups, unsigned long long phase) {
+__device__ __forceinline__ void op_lse_merge(const mdc_mega_params& p, int b, int hq, int n_groups, unsigned long long phase) {
   const mdc_layer_params& L = p.layer;
   n_groups = max(1, min(n_groups, L.H));
   const int nh = ceil_div(L.H, n_groups);
@@ -680,14 +689,97 @@ __device__ inline void op_verify(const mdc_mega_params& p, int src_rank, int slo
 
 namespace mdc {
 
+// The task's body.
+__device__ __forceinline__ void run_task(const mdc_mega_params& p, const CUtensorMap& pages, const TaskInfo& t, unsigned long long phase,
+                                         unsigned char* smem) {
+  const mdc_layer_params& L = p.layer;
+  const int tid = threadIdx.x;
+  const bool worker = tid < kBlockThreads;
+  const bool layer_op = t.op >= MDC_OP_LOGITS && t.op <= MDC_OP_KVWRITE;
+  if (layer_op && (L.B <= 0 || t.c0 < 0 || t.c0 >= L.B)) {  // no (validated) layer behind this queue
+    if (tid == 0) report_failure(p.status, MDC_DEV_BAD_OP, t.op, t.c0, 0, 0);
+  } else
+  switch (t.op) {
+    case MDC_OP_NOP:
+      break;
+    case MDC_OP_LOGITS:
+    {
+      int n;
+      auto run = [&](auto thr) {
+        constexpr bool T = decltype(thr)::value;
+        if (L.logits.fmt == MDC_FMT_MXFP4) return op_logits_call<MDC_FMT_MXFP4, 128, T>(p, &pages, t.c0, t.c1, phase, smem);
+        if (L.logits.page_tokens == 64) {
+          if constexpr (T) return op_logits<MDC_FMT_NVFP4, 64, T>(p, &pages, t.c0, t.c1, phase, smem);
+          else return op_logits_call<MDC_FMT_NVFP4, 64, T>(p, &pages, t.c0, t.c1, phase, smem);
+        }
+        return op_logits_call<MDC_FMT_NVFP4, 128, T>(p, &pages, t.c0, t.c1, phase, smem);
+      };
+      n = row_threshold_fits(L) ? run(std::true_type{}) : run(std::false_type{});
+      if (worker && n >= 0 && L.thr_exact == 4) op_row_fallback(p, t.c0, phase, smem);
+    }
+      break;
+    case MDC_OP_QPATH:
+      if (worker) op_qpath(p, t.c0, t.c1, t.c2, phase, smem);
+      break;
+    case MDC_OP_KVWRITE:
+      if (worker) op_kvwrite(p, t.c0);
+      break;
+    case MDC_OP_MERGE_L1:
+      if (worker) op_merge_l1(p, t.c0, phase, smem);
+      break;
+    case MDC_OP_MERGE_L1A:
+      if (worker && L.mid_v && L.mid_i && L.mid_c) op_merge_l1a(p, t.c0, t.c1, smem);
+      break;
+    case MDC_OP_MERGE_L2:
+      if (worker) {
+        if (L.cp > 1) op_merge_l2<true>(p, t.c0, phase, smem);
+        else op_merge_l2<false>(p, t.c0, phase, smem);
+      }
+      break;
+    case MDC_OP_ATTN:
+      op_attn(p, t.c0, t.c1, t.c2, phase, smem);
+      break;
+    case MDC_OP_LSE_MERGE:
+      if (L.cp > 1) op_lse_merge<true>(p, t.c0, t.c1, t.c2, phase);
+      else op_lse_merge<false>(p, t.c0, t.c1, t.c2, phase);
+      break;
+    case MDC_OP_CMP_STEP:
+    case MDC_OP_CMP_FIN:
+      if (worker) op_cmp(p, t.c0, t.op == MDC_OP_CMP_FIN, phase, smem);
+      break;
+    case MDC_OP_SLEEP:
+      if (tid == 0) {
+        const unsigned long long t0 = global_timer_ns();
+        const unsigned long long want = static_cast<unsigned long long>(min(max(t.c1, 0), 100000000));
+        while (global_timer_ns() - t0 < want) nanosleep(256);
+      }
+      break;
+    case MDC_OP_LOG:
+      if (tid == 0 && p.log) {
+        const int slot = atomicAdd(p.log, 1);
+        if (slot + 1 < p.log_cap) p.log[slot + 1] = t.c0;
+        __threadfence();
+      }
+      break;
+    case MDC_OP_PUSH:
+      if (worker) op_push(p, t.c1, t.c2, phase, smem);
+      break;
+    case MDC_OP_VERIFY:
+      if (worker) op_verify(p, t.c1, t.c2, phase);
+      break;
+    default:
+      if (tid == 0) report_failure(p.status, MDC_DEV_BAD_OP, t.op, t.pos, 0, 0);
+      break;
+  }
+}
+
 __global__ void __launch_bounds__(kMegaThreads, 1) mega_kernel(const __grid_constant__ mdc_mega_params p,
                                                                 const __grid_constant__ CUtensorMap pages) {
   extern __shared__ unsigned char smem_raw[];
+  __shared__ MegaShared sh;
+  const int tid = threadIdx.x;
   wait_for_predecessor();
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  __shared__ MegaShared sh;
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const bool worker = warp < kWarps;
 
   const bool dyn = p.dyn_task_off != nullptr;   // one shared row, tasks pulled with an atomic counter
   const int32_t* row_g = p.queue + (dyn ? 0 : static_cast<int64_t>(blockIdx.x) * p.row_words);
@@ -698,134 +790,72 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_kernel(const __grid_cons
   if (tid == 0) sh.fail = 0;
   __syncthreads();
 
-  Cursor cur;
-  cur.row = staged ? sh.row : row_g;
-  cur.scalars = reinterpret_cast<const unsigned long long*>(p.scalars);
-  cur.arity = p.arity;
-  cur.scopes = p.scopes;
   // The phase is read once per launch.  With phase_ctl set the kernel advances it by itself: every
   // block counts in after its read, and the last one to do so (nobody can read after it) stores
   // phase + 1 for the next launch, so a captured graph replays without a host-side update.
   if (tid == 0) {
-    const unsigned long long ph = ld_acquire_gpu_u64(cur.scalars);
+    const unsigned long long* scalars = reinterpret_cast<const unsigned long long*>(p.scalars);
+    const unsigned long long ph = ld_acquire_gpu_u64(scalars);
     sh.phase = ph;
     if (p.phase_ctl) {
       __threadfence();
       if (atomicAdd(p.phase_ctl, 1ull) + 1ull == static_cast<unsigned long long>(gridDim.x)) {
         *p.phase_ctl = 0ull;
-        *const_cast<volatile unsigned long long*>(cur.scalars) = ph + 1ull;
+        *const_cast<volatile unsigned long long*>(scalars) = ph + 1ull;
       }
     }
   }
   __syncthreads();
-  cur.phase = sh.phase;
   const EventSet ev{static_cast<unsigned char*>(p.events.base), p.events.offsets, p.events.my_rank, p.events.world};
   const mdc_layer_params& L = p.layer;
 
-  TaskInfo t_end;
-  t_end.op = kOpEnd;
-  auto pull = [&]() -> TaskInfo {   // dynamic: the next task of the shared row, or the end marker
+  // Across a task's body only the position of its entry is kept: the rest is read again from shared memory and from the
+  // parameters.  The tiles are functions of their own, and every register that is live across the call is one they
+  // cannot use.
+  auto cursor = [&]() {
+    Cursor c;
+    c.row = staged ? sh.row : row_g;
+    c.scalars = reinterpret_cast<const unsigned long long*>(p.scalars);
+    c.arity = p.arity;
+    c.scopes = p.scopes;
+    c.phase = *const_cast<volatile unsigned long long*>(&sh.phase);
+    return c;
+  };
+  auto pull = [&]() -> int {   // dynamic: the next task of the shared row, or -1
     if (tid == 0) sh.next = static_cast<int32_t>(atomicAdd(p.dyn_ctl, 1u));
     __syncthreads();
     const int idx = sh.next;
     __syncthreads();
-    return idx >= 0 && idx < p.dyn_n_tasks ? cur.read(p.dyn_task_off[idx]) : t_end;
+    return idx >= 0 && idx < p.dyn_n_tasks ? p.dyn_task_off[idx] : -1;
   };
-  for (TaskInfo t = dyn ? pull() : cur.read(0); t.valid(); t = dyn ? pull() : cur.advance(t)) {
-    unsigned long long tr0 = 0, tr1 = 0;
-    if (p.trace && tid == 0) tr0 = global_timer_ns();
-    // ---- waits: thread 0 polls, the barrier publishes
-    if (tid == 0) {
-      if (p.status && *reinterpret_cast<volatile int32_t*>(p.status) != 0) sh.fail = 1;
-      for (int i = 0; i < t.n_waits && !sh.fail; ++i) {
-        const int e = cur.wait_event(t, i);
-        unsigned long long seen = 0;
-        const bool bad_id = e < 0 || e >= p.n_events;
-        if (bad_id || !ev.poll_1t(e, cur.target(e), cur.scopes[e] != 0, p.wait_budget_ns, &seen)) {
-          report_failure(p.status, bad_id ? MDC_DEV_BAD_OP : MDC_DEV_WAIT_TIMEOUT, e, t.op, seen, bad_id ? 0 : cur.target(e));
-          sh.fail = 1;
+  for (int pos = dyn ? pull() : 0; pos >= 0;) {
+    {
+      const Cursor cur = cursor();
+      const TaskInfo t = cur.read(pos);
+      if (!t.valid()) break;
+      // ---- waits: thread 0 polls, the barrier publishes
+      if (tid == 0) {
+        if (p.trace) sh.tr0 = global_timer_ns();
+        if (p.status && *reinterpret_cast<volatile int32_t*>(p.status) != 0) sh.fail = 1;
+        for (int i = 0; i < t.n_waits && !sh.fail; ++i) {
+          const int e = cur.wait_event(t, i);
+          unsigned long long seen = 0;
+          const bool bad_id = e < 0 || e >= p.n_events;
+          if (bad_id || !ev.poll_1t(e, cur.target(e), cur.scopes[e] != 0, p.wait_budget_ns, &seen)) {
+            report_failure(p.status, bad_id ? MDC_DEV_BAD_OP : MDC_DEV_WAIT_TIMEOUT, e, t.op, seen, bad_id ? 0 : cur.target(e));
+            sh.fail = 1;
+          }
         }
+        if (p.trace) sh.tr1 = global_timer_ns();
       }
-    }
-    __syncthreads();
-    if (sh.fail) break;
-    if (p.trace && tid == 0) tr1 = global_timer_ns();
+      __syncthreads();
+      if (sh.fail) break;
 
-    // ---- the task body
-    const bool layer_op = t.op >= MDC_OP_LOGITS && t.op <= MDC_OP_KVWRITE;
-    if (layer_op && (L.B <= 0 || t.c0 < 0 || t.c0 >= L.B)) {  // no (validated) layer behind this queue
-      if (tid == 0) report_failure(p.status, MDC_DEV_BAD_OP, t.op, t.c0, 0, 0);
-    } else
-    switch (t.op) {
-      case MDC_OP_NOP:
-        break;
-      case MDC_OP_LOGITS:
-      {
-        int n;
-        auto run = [&](auto thr) {
-          constexpr bool T = decltype(thr)::value;
-          if (L.logits.fmt == MDC_FMT_MXFP4) return op_logits<MDC_FMT_MXFP4, 128, T>(p, &pages, t.c0, t.c1, cur.phase, smem);
-          if (L.logits.page_tokens == 64) return op_logits<MDC_FMT_NVFP4, 64, T>(p, &pages, t.c0, t.c1, cur.phase, smem);
-          return op_logits<MDC_FMT_NVFP4, 128, T>(p, &pages, t.c0, t.c1, cur.phase, smem);
-        };
-        n = row_threshold_fits(L) ? run(std::true_type{}) : run(std::false_type{});
-        if (worker && n >= 0 && L.thr_exact == 4) op_row_fallback(p, t.c0, cur.phase, smem);
-      }
-        break;
-      case MDC_OP_QPATH:
-        if (worker) op_qpath(p, t.c0, t.c1, t.c2, cur.phase, smem);
-        break;
-      case MDC_OP_KVWRITE:
-        if (worker) op_kvwrite(p, t.c0);
-        break;
-      case MDC_OP_MERGE_L1:
-        if (worker) op_merge_l1(p, t.c0, cur.phase, smem);
-        break;
-      case MDC_OP_MERGE_L1A:
-        if (worker && L.mid_v && L.mid_i && L.mid_c) op_merge_l1a(p, t.c0, t.c1, smem);
-        break;
-      case MDC_OP_MERGE_L2:
-        if (worker) {
-          if (L.cp > 1) op_merge_l2<true>(p, t.c0, cur.phase, smem);
-          else op_merge_l2<false>(p, t.c0, cur.phase, smem);
-        }
-        break;
-      case MDC_OP_ATTN:
-        op_attn(p, t.c0, t.c1, t.c2, cur.phase, smem);
-        break;
-      case MDC_OP_LSE_MERGE:
-        if (L.cp > 1) op_lse_merge<true>(p, t.c0, t.c1, t.c2, cur.phase);
-        else op_lse_merge<false>(p, t.c0, t.c1, t.c2, cur.phase);
-        break;
-      case MDC_OP_CMP_STEP:
-      case MDC_OP_CMP_FIN:
-        if (worker) op_cmp(p, t.c0, t.op == MDC_OP_CMP_FIN, cur.phase, smem);
-        break;
-      case MDC_OP_SLEEP:
-        if (tid == 0) {
-          const unsigned long long t0 = global_timer_ns();
-          const unsigned long long want = static_cast<unsigned long long>(min(max(t.c1, 0), 100000000));
-          while (global_timer_ns() - t0 < want) nanosleep(256);
-        }
-        break;
-      case MDC_OP_LOG:
-        if (tid == 0 && p.log) {
-          const int slot = atomicAdd(p.log, 1);
-          if (slot + 1 < p.log_cap) p.log[slot + 1] = t.c0;
-          __threadfence();
-        }
-        break;
-      case MDC_OP_PUSH:
-        if (worker) op_push(p, t.c1, t.c2, cur.phase, smem);
-        break;
-      case MDC_OP_VERIFY:
-        if (worker) op_verify(p, t.c1, t.c2, cur.phase);
-        break;
-      default:
-        if (tid == 0) report_failure(p.status, MDC_DEV_BAD_OP, t.op, t.pos, 0, 0);
-        break;
+      run_task(p, pages, t, cur.phase, smem);
     }
-
+    asm volatile("" ::: "memory");
+    const Cursor cur = cursor();
+    const TaskInfo t = cur.read(pos);
     // ---- notifies: everything this block wrote is released first
     // (threads that issued bulk copies have completed them and fenced the async proxy inside the
     // op; the barrier orders every thread's writes before thread 0's fence, which is cumulative, so
@@ -851,12 +881,13 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_kernel(const __grid_cons
         unsigned long long* e = p.trace + 4 + 4 * slot;
         e[0] = (static_cast<unsigned long long>(blockIdx.x) << 32) | (static_cast<unsigned long long>(t.op & 0xff) << 24) |
                (static_cast<unsigned long long>(t.c0 & 0xfff) << 12) | static_cast<unsigned long long>(t.c1 & 0xfff);
-        e[1] = tr0;
-        e[2] = tr1;
+        e[1] = sh.tr0;
+        e[2] = sh.tr1;
         e[3] = global_timer_ns();
       }
     }
     __syncthreads();
+    pos = dyn ? pull() : pos + 4 + t.n_waits + t.n_notifies;
   }
   if (dyn && tid == 0) {   // the last block to finish rewinds the counters for the next launch
     __threadfence();

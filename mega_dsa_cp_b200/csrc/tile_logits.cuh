@@ -3,46 +3,36 @@
 // writes the fp32 logits row or keeps the chunk's scores in shared memory and
 // emits the exact local top-k.
 //
-// The tile is a four-role pipeline over 128-token stages, handed on in pairs:
+// Four groups of four warps take the 128-token stages in turn, each with tensor memory, a slot pair of the raw ring
+// and barriers of its own:
 //
-//   copy warp          a page is contiguous in HBM (P x 64 B of packed E2M1,
-//                      then the page's block scales); one tiled TMA load per page
-//                      fills a ring of 8 raw stages in shared memory and swizzles
-//                      its 64-byte rows on the way (16-byte chunk j of row r at
-//                      j ^ (r / 2 % 4)), which is what makes the row loads below
-//                      bank-conflict free.  Lane l owns one page slot of the ring;
-//                      the lanes poll the "empty" barriers of their stages
-//                      together and refill whatever is free.
-//   decode warps (0-7) two groups of four warps take the even and the odd pairs
-//                      of stages.  Thread i of a group owns token row i of both: it
-//                      reads 64 B of codes (four 16-byte loads) and the scales of
-//                      each, converts with cvt.f16x2.e2m1x2, multiplies by the block
-//                      scale (exact in fp16) and stores the row into TENSOR MEMORY
-//                      (tcgen05.st) as the A operand of the stage's MMA; a ring of
-//                      two A pairs.
-//   issue warp(s)      one thread of each issues eight tcgen05.mma (M=128 tokens,
-//                      N=64*q_len heads, K=16, fp16 x fp16 -> fp32) per stage,
-//                      A from tensor memory, B = the query block, staged once
-//                      in shared memory in the K-major 128-byte-swizzle layout;
-//                      two accumulator pairs (q_len 1) or stages in tensor memory.
-//   gate warps         GG groups of four warps take pairs (stages) round-robin; thread
-//                      i reads accumulator row i of both stages (tcgen05.ld), applies
-//                      relu and the head weights, reduces over heads and emits the
-//                      tokens' scores.
+//   copy     a page is contiguous in HBM (P x 64 B of packed E2M1, then the page's block scales); one tiled TMA load
+//            per page fills a raw stage in shared memory and swizzles its 64-byte rows on the way (16-byte chunk j of
+//            row r at j ^ (r / 2 % 4)), which is what makes the row loads below bank-conflict free.  The group that
+//            has read a stage loads the stage kRawStages further on into it.
+//   decode   thread i of a group owns token row i: it reads 64 B of codes (four 16-byte loads) and the row's scales,
+//            converts with cvt.f16x2.e2m1x2, multiplies by the block scale (exact in fp16) and stores the row into
+//            TENSOR MEMORY (tcgen05.st) as the A operand.
+//   product  behind a barrier of the group's 128 threads one of them issues eight tcgen05.mma (M=128 tokens, N=64
+//            heads, K=16, fp16 x fp16 -> fp32) per query token, B = the query block, staged once in shared memory in
+//            the K-major 128-byte-swizzle layout.
+//   gate     while it runs, the group takes the accumulator row that it has read (tcgen05.ld) before issuing it: relu,
+//            head weights, sum over heads, the scores of the stage (or query token) before.
 //
 // Keeping A in tensor memory instead of shared memory matters: the decode
 // output (32 KB per stage) and its re-read by the tensor core would otherwise
 // triple the shared-memory traffic of a kernel that has to sustain one stage
 // per ~400 cycles to follow HBM.
 //
-// What bounds the loop is issue slots and the latency of each hand-off (an mbarrier
-// probe or a shared-memory atomic costs a warp 100-200 cycles even when it succeeds
-// at once).  Hence pairs: two rows per thread and hand-off keep twice the
-// independent work in flight and halve the hand-offs, and the gate reads its
-// weights once for two rows.  Measured on 37 sequences x 16384 tokens (NVFP4, 32
-// stages per SM, logits out): 20.0 -> 18.4 us, of which about 6 us do not
-// depend on the length (launch, prologue, fill and drain); three decode groups, three or
-// four gate groups, one gate group, a ring of 12 or 16 raw stages: slower or equal.
+// What bounds the loop is latency between dependent steps and instruction fetch, with every pipe half used (ALU, shared
+// memory, issue slots and tensor core each need 250-400 cycles per stage).  So the groups share nothing: no counters or
+// barriers between producer and consumer warps, no warp that only polls; a group's step waits for its raw stage and for
+// its own product, both of which have had most of a step to complete.  The form before had two decode groups, two gate
+// groups, two issue warps and a copy warp (one gate group and one issue warp in the persistent kernel), handing stages on
+// in pairs.  32 x 32768 tokens with row top-k 38.9 -> 36.0 us, 37 sequences x 16384 tokens, logits out, 18.0 -> 15.4,
+// two query tokens, 16 x 32768 MXFP4, 32.2 -> 29.0, 3 x 20032 6.4 -> 5.1 (of which the query's loads in flight together
+// 1.0), the persistent kernel's step of 8 x 131072 84.6 -> 79.1.  Three groups, with issue and copy warps: 43.5 for the
+// first of these; the warps of a group taking turns to issue: 37.7.
 //
 // Exactness.  K values (E2M1 x scale) are exact in fp16.  Query rows are
 // rescaled per head by a power of two so that the largest element lands in
@@ -70,17 +60,12 @@ namespace mdc {
 constexpr int kIdxDim = 128;
 constexpr int kIdxHeads = 64;
 constexpr int kTileTok = 128;    // tokens per pipeline stage (= UMMA M)
-constexpr int kRawStages = 8;    // raw page ring
-constexpr int kAStages = 4;      // decoded-A ring in tensor memory: two pairs
-constexpr int kTmemCols = 512;
+constexpr int kLogitsGroups = 4; // groups of four warps; 512 threads leave each 128 registers
+constexpr int kRawStages = 8;    // raw page ring: two slots per group
+constexpr int kTmemCols = 512;   // per group 64 columns of accumulator (128 rows x 64 heads) and 64 of decoded A
 constexpr int kFusedRegE = 32;   // fused top-k keeps up to 256 * 32 scores per query token in registers
-
-// Warp layout for DG decode groups, GG gate groups and NI issue warps: 4*DG decode, 4*GG gate, NI issue, 1 copy.
-constexpr int logits_threads(int dg, int gg, int ni) { return (4 * dg + 4 * gg + ni + 1) * 32; }
-// The stand-alone kernel.  Two issue warps take the stages in turn: one alone spends as long between the MMAs of two
-// stages as on issuing them (37 sequences x 16384 tokens, logits out: 20.7 us with one, 19.1 with two).
-constexpr int kLogitsDecodeGroups = 2, kLogitsGateGroups = 2, kLogitsIssueWarps = 2;
-constexpr int kLogitsThreads = logits_threads(kLogitsDecodeGroups, kLogitsGateGroups, kLogitsIssueWarps);
+constexpr int kLogitsThreads = kLogitsGroups * 128;
+static_assert(kRawStages % kLogitsGroups == 0 && kLogitsGroups * 128 <= kTmemCols, "slots and columns of the groups");
 
 template <int FMT, int PAGE>
 struct IdxPage {
@@ -91,7 +76,7 @@ struct IdxPage {
   static constexpr int kStageBytes = kTilePages * kBytes;
   static constexpr int kRows = kBytes / 64;   // a page as 64-byte rows: the tensor map's box
   static_assert(kBytes % 512 == 0 && kRows <= 256, "the 64-byte swizzle repeats every 512 bytes");
-  // byte offset o of a page lies here after the copy's swizzle
+  // byte offset o of a page lies here after the copy's swizzle (a page starts on a 512-byte boundary)
   __device__ static int swizzled(int o) { return o ^ ((o >> 3) & 0x30); }
 };
 
@@ -119,8 +104,8 @@ __host__ __device__ constexpr LogitsSmem logits_smem_layout(int q_len, int chunk
   off += kRawStages * IdxPage<FMT, PAGE>::kStageBytes;
   off = static_cast<int>(align_up(off, 128));
   L.bars = off;
-  off += (2 * kRawStages + kAStages) * 8;
-  L.misc = off;  // [0] tensor-memory base, [1] abort flag, [4..9] and [10..11] progress counters
+  off += (kRawStages + kLogitsGroups) * 8;
+  L.misc = off;  // [0] tensor-memory base, [1] abort flag, [12..13] selected
   off += 64;
   L.wsc = off;
   off += q_len * kIdxHeads * 4;
@@ -135,7 +120,7 @@ __host__ __device__ constexpr LogitsSmem logits_smem_layout(int q_len, int chunk
   L.scores = off;
   if (fused) off += q_len * chunk_tokens * 4;
   off = static_cast<int>(align_up(off, 16));
-  L.hist = off;  // histograms of the chunk's keys, one per query token, filled by the gate warps
+  L.hist = off;  // histograms of the chunk's keys, one per query token, filled with the scores
   if (hist) off += q_len * MDC_THR_BINS * 4;
   L.total = static_cast<int>(align_up(off, 128));
   return L;
@@ -157,59 +142,72 @@ template <int T>
 __device__ inline void logits_stage_query(const mdc_logits_params& p, int b, unsigned char* qb, float* wsc) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int hl = lane & 15, sub = lane >> 4;
-  constexpr int N = T * kIdxHeads;
-  for (int row0 = warp * 2; row0 < N; row0 += kWarps * 2) {
-    const int row = row0 + sub;
-    float v[8];
-    if (p.q_fmt == MDC_Q_BF16) {
-      const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(p.q) +
-                                 (static_cast<int64_t>(b) * N + row) * kIdxDim + 8 * hl;
-      uint4 raw = *reinterpret_cast<const uint4*>(src);
-      const uint32_t w4[4] = {raw.x, raw.y, raw.z, raw.w};
+  constexpr int N = T * kIdxHeads, kBatch = 4;   // rows of a half-warp whose loads are in flight together
+  static_assert(N % (kWarps * 2 * kBatch) == 0, "whole batches");
+#pragma unroll 1
+  for (int row0 = warp * 2 + sub; row0 < N; row0 += kWarps * 2 * kBatch) {
+    uint4 raw[kBatch];
+    float w[kBatch];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        v[2 * i] = __uint_as_float(w4[i] << 16);
-        v[2 * i + 1] = __uint_as_float(w4[i] & 0xffff0000u);
+    for (int k = 0; k < kBatch; ++k) {
+      const int row = row0 + k * kWarps * 2;
+      const int64_t at = static_cast<int64_t>(b) * N + row;
+      if (p.q_fmt == MDC_Q_BF16) {
+        raw[k] = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.q) + at * kIdxDim + 8 * hl);
+      } else {
+        raw[k].x = *reinterpret_cast<const uint32_t*>(static_cast<const uint8_t*>(p.q) + at * 64 + 4 * hl);
+        // atom-ordered scales: 512 B per block of 128 rows
+        const uint8_t* sfb = p.q_sf + static_cast<int64_t>(b) * ceil_div(N, 128) * 512 + (row / 128) * 512;
+        const int r = row % 128;
+        raw[k].y = sfb[(r % 32) * 16 + (r / 32) * 4 + hl / 4];
       }
-    } else {
-      const uint8_t* src = static_cast<const uint8_t*>(p.q) + (static_cast<int64_t>(b) * N + row) * 64 + 4 * hl;
-      const uint32_t eight = *reinterpret_cast<const uint32_t*>(src);
-      // atom-ordered scales: 512 B per block of 128 rows
-      const uint8_t* sfb = p.q_sf + static_cast<int64_t>(b) * ceil_div(N, 128) * 512 + (row / 128) * 512;
-      const int r = row % 128;
-      const uint32_t e = sfb[(r % 32) * 16 + (r / 32) * 4 + hl / 4];
-      const float sc = __uint_as_float(e << 23);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = e2m1_to_float((eight >> (4 * i)) & 0xf) * sc;
+      w[k] = p.weights[at];
     }
-    float m = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(v[i]));
+    for (int k = 0; k < kBatch; ++k) {
+      const int row = row0 + k * kWarps * 2;
+      float v[8];
+      if (p.q_fmt == MDC_Q_BF16) {
+        const uint32_t w4[4] = {raw[k].x, raw[k].y, raw[k].z, raw[k].w};
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    // power-of-two rescale: bring the largest magnitude to [2^14, 2^15)
-    int ex = static_cast<int>((__float_as_uint(m) >> 23) & 0xff) - 127;
-    int up = 14 - ex;
-    up = max(-100, min(100, up));
-    if (m == 0.f || !(m < 3.0e38f)) up = 0;
-    const float scale = __uint_as_float(static_cast<uint32_t>(127 + up) << 23);
-    const float inv = __uint_as_float(static_cast<uint32_t>(127 - up) << 23);
-    uint4 out;
-    {
-      __half2 h0 = __floats2half2_rn(v[0] * scale, v[1] * scale);
-      __half2 h1 = __floats2half2_rn(v[2] * scale, v[3] * scale);
-      __half2 h2 = __floats2half2_rn(v[4] * scale, v[5] * scale);
-      __half2 h3 = __floats2half2_rn(v[6] * scale, v[7] * scale);
-      out.x = *reinterpret_cast<uint32_t*>(&h0);
-      out.y = *reinterpret_cast<uint32_t*>(&h1);
-      out.z = *reinterpret_cast<uint32_t*>(&h2);
-      out.w = *reinterpret_cast<uint32_t*>(&h3);
+        for (int i = 0; i < 4; ++i) {
+          v[2 * i] = __uint_as_float(w4[i] << 16);
+          v[2 * i + 1] = __uint_as_float(w4[i] & 0xffff0000u);
+        }
+      } else {
+        const float sc = __uint_as_float(raw[k].y << 23);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = e2m1_to_float((raw[k].x >> (4 * i)) & 0xf) * sc;
+      }
+      float m = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(v[i]));
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      // power-of-two rescale: bring the largest magnitude to [2^14, 2^15)
+      int ex = static_cast<int>((__float_as_uint(m) >> 23) & 0xff) - 127;
+      int up = 14 - ex;
+      up = max(-100, min(100, up));
+      if (m == 0.f || !(m < 3.0e38f)) up = 0;
+      const float scale = __uint_as_float(static_cast<uint32_t>(127 + up) << 23);
+      const float inv = __uint_as_float(static_cast<uint32_t>(127 - up) << 23);
+      uint4 out;
+      {
+        __half2 h0 = __floats2half2_rn(v[0] * scale, v[1] * scale);
+        __half2 h1 = __floats2half2_rn(v[2] * scale, v[3] * scale);
+        __half2 h2 = __floats2half2_rn(v[4] * scale, v[5] * scale);
+        __half2 h3 = __floats2half2_rn(v[6] * scale, v[7] * scale);
+        out.x = *reinterpret_cast<uint32_t*>(&h0);
+        out.y = *reinterpret_cast<uint32_t*>(&h1);
+        out.z = *reinterpret_cast<uint32_t*>(&h2);
+        out.w = *reinterpret_cast<uint32_t*>(&h3);
+      }
+      // dims 8*hl .. 8*hl+7: K-half = hl / 8, 16-byte chunk = hl % 8
+      unsigned char* dst = qb + (hl >> 3) * (N * 128) + row * 128 + (((hl & 7) ^ (row & 7)) << 4);
+      *reinterpret_cast<uint4*>(dst) = out;
+      // 0.5 for the (x + |x|) form of relu
+      if (hl == 0) wsc[row] = 0.5f * w[k] * inv;
     }
-    // dims 8*hl .. 8*hl+7: K-half = hl / 8, 16-byte chunk = hl % 8
-    unsigned char* dst = qb + (hl >> 3) * (N * 128) + row * 128 + (((hl & 7) ^ (row & 7)) << 4);
-    *reinterpret_cast<uint4*>(dst) = out;
-    // 0.5 for the (x + |x|) form of relu
-    if (hl == 0) wsc[row] = 0.5f * p.weights[static_cast<int64_t>(b) * N + row] * inv;
   }
 }
 
@@ -825,7 +823,7 @@ static __device__ __noinline__ bool chunk_publish_row_one_rank(const RowThreshol
   return true;
 }
 
-// hs: the chunk's histogram, already filled (the gate warps count their keys into it), keys: the chunk's keys.  scratch: the
+// hs: the chunk's histogram, already filled, keys: the chunk's keys.  scratch: the
 // raw ring, idle by now.
 template <typename Emit>
 __device__ inline int chunk_emit_above_row_threshold(const RowThreshold& rt, int32_t* status, int b, int chunk, int n_chunks,
@@ -1200,47 +1198,39 @@ __device__ void logits_row_select(const mdc_logits_params& p, int b, int chunk, 
   }
 }
 
-// The tile.  smem: dynamic shared memory base (1024 B aligned), laid out by
-// logits_smem_layout.  All logits_threads(GG) threads of the block call it.
-// Returns, to the worker threads alike, the entries of the (last) candidate list, or -1 when the row has been published or
-// nothing was written.
-template <int FMT, int PAGE, int T, int DG, int GG, int NI, bool ROWK = false>
-__device__ __forceinline__ int logits_tile(const mdc_logits_params& p, const CUtensorMap* pages, int b, int chunk, unsigned char* smem,
-                           const RowThreshold* rt = nullptr) {
+// Whether the chunk's scores are kept as sortable keys and counted: for a row threshold, and in the stand-alone kernels where
+// they fit.
+template <int FMT, int PAGE, int T, bool ALONE, bool THR>
+__device__ __forceinline__ bool logits_keeps_keys(bool fused, int chunk_tokens) {
+  return ALONE ? fused && logits_as_keys<FMT, PAGE>(T, chunk_tokens) : THR;
+}
+
+// Scores the chunk.  smem: dynamic shared memory base (1024 B aligned), laid out by logits_smem_layout.  All threads of the
+// block call it.  ALONE: the stand-alone kernels; THR: the persistent kernel with a row threshold, `hist_next`: the row's
+// histogram of the next step, of which this task zeroes its slice.  Returns the chunk's pages, or their complement (< 0) when
+// a wait ran out.
+template <int FMT, int PAGE, int T, bool ALONE, bool ROWK, bool THR>
+__device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const CUtensorMap* pages, int b, int chunk, unsigned char* smem,
+                                             uint32_t* hist_next) {
   using PG = IdxPage<FMT, PAGE>;
   constexpr int N = T * kIdxHeads;
-  constexpr int kThreads = logits_threads(DG, GG, NI);
-  constexpr int kGateWarp0 = 4 * DG, kIssueWarp = kGateWarp0 + 4 * GG, kCopyWarp = kIssueWarp + NI;
-  // Tensor memory: 256 accumulator columns (two pairs of stages at q_len 1, two single stages at q_len 2), then
-  // two pairs of decoded-A stages of 64 columns (128 fp16 per row).
-  constexpr bool kAccPairs = T == 1;
-  constexpr int kAccSt = 256 / N, kAPairs = kAStages / 2, kASt = kAStages;
-  constexpr uint32_t kAccBase = 0, kABase = kAccSt * N;
-  static_assert(kABase + kASt * 64 <= kTmemCols && kASt <= kAStages, "tensor memory over-subscribed");
-  static_assert(kRawStages * PG::kTilePages <= 32, "one copy-warp lane per page of the raw ring");
+  constexpr int G = kLogitsGroups, kThreads = kLogitsThreads;
+  constexpr int kCopyWarp = kWarps, kTmemWarp = kWarps + 1;   // set-up: the first ring fill and the barriers; tensor memory
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const bool row_mode = ROWK && p.row_v != nullptr;
-  const bool fused = p.cand_v != nullptr || row_mode;
+  const bool fused = p.cand_v != nullptr || (ROWK && p.row_v != nullptr);
   const int chunk_tokens = p.blocks_per_chunk * PAGE;
-  // the gate warps keep sortable keys and count them: for a row threshold, and in the stand-alone kernel (its two gate
-  // groups) where they fit
-  constexpr bool kAlone = GG == kLogitsGateGroups;   // (what only it does is compiled for it alone)
-  const bool as_keys = kAlone ? fused && logits_as_keys<FMT, PAGE>(T, chunk_tokens) : rt != nullptr;
+  const bool as_keys = logits_keeps_keys<FMT, PAGE, T, ALONE, THR>(fused, chunk_tokens);
   const LogitsSmem L = logits_smem_layout<FMT, PAGE>(T, chunk_tokens, fused, as_keys);
   uint32_t* hs = reinterpret_cast<uint32_t*>(smem + L.hist);
 
   unsigned char* qb = smem + L.qb;
   unsigned char* ring = smem + L.ring;
   uint64_t* raw_full = reinterpret_cast<uint64_t*>(smem + L.bars);
-  uint64_t* raw_empty = raw_full + kRawStages;
-  uint64_t* mma_done = raw_empty + kRawStages;  // [kAStages]: stage t finished on the tensor core (slot t % kASt)
+  uint64_t* mma_done = raw_full + kRawStages;   // [G]: the group's product is complete
   uint32_t* misc = reinterpret_cast<uint32_t*>(smem + L.misc);
   volatile uint32_t* abort_flag = misc + 1;
-  uint32_t* a_cnt = misc + 4;    // [kAPairs] decode warps that finished writing the A pair (monotonic)
-  uint32_t* acc_cnt = misc + 10;  // [2] gate warps that finished reading the accumulator pair / stage (monotonic)
   int32_t* page_id = reinterpret_cast<int32_t*>(smem + L.page_ok);
   float* wsc = reinterpret_cast<float*>(smem + L.wsc);
-  SelectScratch& sel = *reinterpret_cast<SelectScratch*>(smem + L.sel);
   float* scores = reinterpret_cast<float*>(smem + L.scores);
 
   const int blk0 = chunk * p.blocks_per_chunk;
@@ -1252,68 +1242,67 @@ __device__ __forceinline__ int logits_tile(const mdc_logits_params& p, const CUt
   if (fused) blk_end = min(blk_end, ceil_div(limit, PAGE));
   const int n_pages = max(0, blk_end - blk0);
   const int n_tiles = ceil_div(n_pages, PG::kTilePages);  // pipeline stages of this block
-  const int n_pairs = ceil_div(n_tiles, 2);
   const int32_t* bt = p.block_table + static_cast<int64_t>(b) * p.max_pages;
+  const int table_end = min(p.blocks_per_chunk, p.max_pages - blk0);   // the chunk's entries of the page table
+  int bad_page = 0;
   constexpr long long kBudget = 1ll << 31;  // clock cycles a role waits before it gives up
 
-  // ---------------- prologue.  The copy warp fills the ring at once; the query, the page table and tensor memory are
+  // ---------------- prologue.  One warp fills the ring at once; the query, the page table and tensor memory are
   // set up meanwhile.
   const uint64_t stream_policy = l2_policy_evict_first();  // the index cache is read once per step
-  const int cs = lane / PG::kTilePages, cp = lane % PG::kTilePages;   // copy warp: lane l owns page cp of raw stage cs
-  // The lanes of a stage load tile `tile` into it: id = the lane's page (-1 = none).
-  auto refill = [&](bool go, int id) {
-    const uint32_t bytes_all = __ballot_sync(0xffffffffu, id >= 0);
-    const int n = __popc((bytes_all >> (lane - cp)) & ((1u << PG::kTilePages) - 1u));
-    if (!go) return;
-    if (cp == 0) {
+  // Loads page `id` (-1 = none) into page slot cp of raw stage cs; one lane per page, the lanes of a stage next to each other
+  // (cp = lane % pages of a stage).  `go`: alike in the lanes of a stage.
+  auto refill = [&](bool go, int cs, int cp, int id) {
+    const uint32_t there = __ballot_sync(0xffffffffu, id >= 0);
+    const int n = __popc((there >> (lane - cp)) & ((1u << PG::kTilePages) - 1u));
+    if (go && cp == 0) {
       if (n == 0) mbar_arrive(&raw_full[cs]);
       else mbar_expect_tx(&raw_full[cs], static_cast<uint32_t>(n) * PG::kBytes);
     }
-    __syncwarp(__activemask());
-    if (id >= 0) tma_load_3d_hint(ring + cs * PG::kStageBytes + cp * PG::kBytes, pages, 0, 0, id, &raw_full[cs], stream_policy);
+    __syncwarp();
+    if (go && id >= 0)
+      tma_load_3d_hint(ring + cs * PG::kStageBytes + cp * PG::kBytes, pages, 0, 0, id, &raw_full[cs], stream_policy);
   };
   if (warp == kCopyWarp) {
     if (lane == 0) {
-      for (int s = 0; s < kRawStages; ++s) {
-        mbar_init(&raw_full[s], 1);
-        mbar_init(&raw_empty[s], 4);
-      }
-      for (int s = 0; s < kAStages; ++s) mbar_init(&mma_done[s], 1);
+      for (int s = 0; s < kRawStages + G; ++s) mbar_init(&raw_full[s], 1);
       for (int i = 1; i < 16; ++i) misc[i] = 0;
       mbar_fence_init();
     }
     fence_proxy_async_smem();   // (the ring may have been the previous task's scratch)
     __syncwarp();
-    int id = lane < n_pages ? bt[blk0 + lane] : -1;
-    if (id >= p.num_pages) id = -1;
-    refill(cs < kRawStages && cs < n_tiles, id);
+    // (read up to the chunk's end: the load does not wait for the sequence's length)
+    int id = lane < table_end ? bt[blk0 + lane] : -1;
+    if (lane >= n_pages || id >= p.num_pages) id = -1;
+    refill(lane < min(kRawStages, n_tiles) * PG::kTilePages, lane / PG::kTilePages, lane % PG::kTilePages, id);
   } else if (warp < kWarps) {
     logits_stage_query<T>(p, b, qb, wsc);
     fence_proxy_async_smem();  // the tensor core reads the query block through the async proxy
   } else {
-    if (warp == kIssueWarp) umma::tmem_alloc(misc, kTmemCols);
+    if (warp == kTmemWarp) umma::tmem_alloc(misc, kTmemCols);
     if (as_keys) {
-      const int t = tid - kBlockThreads, nt = kThreads - kBlockThreads - 32;
+      const int t = tid - kBlockThreads - (warp > kCopyWarp ? 32 : 0), nt = kThreads - kBlockThreads - 32;
       for (int i = t; i < T * kThrBins / 4; i += nt) reinterpret_cast<uint4*>(hs)[i] = make_uint4(0u, 0u, 0u, 0u);
-      if (rt) {  // this task's slice of the next step's histogram
+      if (THR) {  // this task's slice of the next step's histogram
         const int per = ceil_div(kThrBins, p.n_chunks), end = min(kThrBins, (chunk + 1) * per);
-        for (int i = chunk * per + t; i < end; i += nt) rt->hist_next[static_cast<int64_t>(b) * kThrBins + i] = 0u;
+        for (int i = chunk * per + t; i < end; i += nt) hist_next[i] = 0u;
       }
     }
-    for (int i = tid - kBlockThreads; i < n_pages + 4; i += kThreads - kBlockThreads - 32) {  // (+4: the slots behind the last page read as unusable)
-      int32_t id = -1;
-      if (i < n_pages) {
-        id = bt[blk0 + i];
-        if (id < 0 || id >= p.num_pages) {
-          report_failure(p.status, MDC_DEV_BAD_INDEX, id, blk0 + i, 0, 0);
-          id = -1;
-        }
+    const int t = tid - kBlockThreads - (warp > kCopyWarp ? 32 : 0);
+    for (int i = t; i < table_end + 4; i += kThreads - kBlockThreads - 32) {  // (+4: the slots behind the last page)
+      int32_t id = i < table_end ? bt[blk0 + i] : -1;
+      if (i >= n_pages) {
+        id = -1;
+      } else if (id < 0 || id >= p.num_pages) {
+        report_failure(p.status, MDC_DEV_BAD_INDEX, id, blk0 + i, 0, 0);
+        id = -1;
+        bad_page = 1;
       }
       page_id[i] = id;
     }
   }
   umma::fence_before_sync();
-  __syncthreads();
+  const bool any_bad = __syncthreads_or(bad_page) != 0;
   umma::fence_after_sync();
   const uint32_t tmem = misc[0];
   const float neg_inf = __int_as_float(0xff800000);
@@ -1322,128 +1311,97 @@ __device__ __forceinline__ int logits_tile(const mdc_logits_params& p, const CUt
     report_failure(p.status, MDC_DEV_COPY_TIMEOUT, what, idx, 0, 0);
     *abort_flag = 1;
   };
-  // Waits for the MMAs of stage t and, with `two`, of stage t + 1 (one issue warp: the later implies the earlier).
-  auto stages_done = [&](int t, bool two) -> bool {
-    auto done = [&](int i) { return mbar_wait(&mma_done[i % kASt], (i / kASt) & 1, kBudget, abort_flag); };
-    if (NI == 1) return done(t + (two ? 1 : 0));
-    return done(t) && (!two || done(t + 1));
-  };
-
-  if (warp == kCopyWarp) {
-    // ---------------- copy warp.  The lanes poll their stages' "empty" barriers together without blocking and every
-    // lane whose stage is free issues its page's copy in the same instruction, so the ring is
-    // refilled in whatever order the decode warps release it and no single thread serialises
-    // the address arithmetic of all pages.
-    int tile = cs < kRawStages ? cs + kRawStages : n_tiles;
-    long long t_last = clock64();
-    while (__any_sync(0xffffffffu, tile < n_tiles) && !*abort_flag) {
-      bool ready = false;
-      if (tile < n_tiles) ready = mbar_test(&raw_empty[cs], ((tile / kRawStages) - 1) & 1);
-      ready = __shfl_sync(0xffffffffu, ready, lane - cp);  // the lanes of a stage act on one answer
-      refill(ready, ready ? page_id[tile * PG::kTilePages + cp] : -1);
-      if (ready) tile += kRawStages;
-      __syncwarp();
-      if (__any_sync(0xffffffffu, ready)) {
-        t_last = clock64();
-        continue;
-      }
-      __nanosleep(200);  // nothing to refill: do not spin hot beside the decode warps
-      if (clock64() - t_last > kBudget) {
-        if (lane == 0) give_up(0, tile);
-        break;
-      }
-    }
-  } else if (warp >= kIssueWarp && warp < kCopyWarp) {
-    // ---------------- issue warp: all lanes walk the loop together, one elected lane issues
-    // (the tensor-core instructions take warp-uniform operands)
-    constexpr uint32_t idesc = umma::idesc_f16(kTileTok, N, 0);
-    const uint32_t qb_u = smem_u32(qb);
-    uint64_t bdesc[8];
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk) bdesc[kk] = umma::smem_desc_sw128(qb_u + (kk >> 2) * (N * 128) + (kk & 3) * 32);
-    auto wait_or_leave = [&](const uint32_t* cnt, uint32_t target, int tile) -> bool {
-      // progress counters instead of mbarriers here: an mbarrier wait costs this
-      // thread ~150 cycles even when the phase is long complete
-      const bool ok = counter_wait(cnt, target, kBudget, abort_flag);
-      if (__all_sync(0xffffffffu, ok)) return true;
-      if (lane == 0) give_up(1, tile);
-      return false;
-    };
-    for (int tile = warp - kIssueWarp; tile < n_tiles; tile += NI) {
-      const int a = tile % kASt, c = tile % kAccSt, pair = tile >> 1;
-      const int h = kAccPairs ? pair : tile;   // hand-off to the gate warps
-      const bool first = NI > 1 || (tile & 1) == 0;   // of its pair, for this warp
-      if (first && !wait_or_leave(&a_cnt[pair % kAPairs], 4u * (pair / kAPairs + 1), tile)) break;
-      if ((first || !kAccPairs) && h >= 2 && !wait_or_leave(&acc_cnt[h & 1], 4u * (h / 2), tile)) break;
-      umma::fence_after_sync();
-      if (umma::elect_one()) {
-        umma::mma_f16_ts_x8(tmem + kAccBase + c * N, tmem + kABase + a * 64, bdesc, idesc);
-        umma::commit(&mma_done[a]);
-      }
-      __syncwarp();
-    }
-  } else if (warp < kGateWarp0) {
-    // ---------------- decode warps: thread = token row; group g (warps 4g..4g+3) takes the pairs g, g + DG, ...
+  {
+    // ---------------- the groups: thread = token row; group g (warps 4g..4g+3) takes the stages g, g + G, ...
     const int quad = warp & 3, grp = warp >> 2;  // TMEM lane quadrant, group
     const int row = quad * 32 + lane;
     const int pp = row / PAGE, tok = row % PAGE;
-    const uint32_t t_row = tmem + (static_cast<uint32_t>(quad * 32) << 16) + kABase;
-    int code_at[4];   // the row's 16-byte chunks inside its stage
-#pragma unroll
-    for (int j = 0; j < 4; ++j) code_at[j] = pp * PG::kBytes + PG::swizzled(tok * 64 + 16 * j);
-    const int sf_at = pp * PG::kBytes +
-                      PG::swizzled(PG::kData + (FMT == MDC_FMT_NVFP4 ? tok * 8 : (tok % 32) * 16 + (tok / 32) * 4));
-    for (int pair = grp; pair < n_pairs; pair += DG) {
-      const int t0 = 2 * pair;
-      const bool two = t0 + 1 < n_tiles;
-      uint4 d[2][4];
-      uint2 raw_sf[2];  // the rows' block scales
-      bool fine = true;
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int tile = t0 + k, s = tile % kRawStages;
-        const bool there = k == 0 || two;
-        if (there && fine && !mbar_wait(&raw_full[s], (tile / kRawStages) & 1, kBudget, abort_flag)) {
+    const uint32_t t_acc = tmem + grp * 64, t_a = tmem + (G + grp) * 64;
+    const uint32_t t_lane = static_cast<uint32_t>(quad * 32) << 16;
+    const int row_at = pp * PG::kBytes + tok * 64, turn = (tok * 8) & 0x30;   // the row in its stage: chunk j at (16 j) ^ turn
+    const int sf_at = PG::swizzled(PG::kData + (FMT == MDC_FMT_NVFP4 ? tok * 8 : (tok % 32) * 16 + (tok / 32) * 4)) - tok * 64;   // from there
+    const int n_here = n_pages * PAGE, n_cand = limit - blk0 * PAGE;   // positions that exist; that can be selected
+    auto emit = [&](int local, int t, float score) {   // local: position inside the chunk
+      if (local < n_here) {
+        float val = score;
+        if (any_bad && page_id[local / PAGE] < 0) val = neg_inf;
+        if (as_keys) {   // 0 = not a candidate
+          const uint32_t key = local < n_cand ? max(sortable_u32(val), 1u) : 0u;
+          reinterpret_cast<uint32_t*>(scores)[t * chunk_tokens + local] = key;
+          if (key) atomicAdd(&hs[t * kThrBins + (key >> kThrShift)], 1u);
+        } else if (fused) scores[t * chunk_tokens + local] = val;
+        else p.logits[(static_cast<int64_t>(b) * T + t) * p.logits_stride + static_cast<int64_t>(blk0) * PAGE + local] = val;
+      }
+    };
+    constexpr uint32_t idesc = umma::idesc_f16(kTileTok, kIdxHeads, 0);
+    const uint32_t qb_u = smem_u32(qb);
+    // Step n of the group: the product of stage grp + G * (n / T) and query token n % T is issued, the scores of step n - 1
+    // are computed.  A wait that runs out leaves the loop's barriers in place: every warp of the group walks them all.
+    // (The tensor-memory loads stand outside the conditions, the first step's read nothing of use: inside the persistent
+    // kernel conditional ones made every function of it spill.)
+    const int steps = n_tiles > grp ? ceil_div(n_tiles - grp, G) * T : 0;
+    bool ok = true;
+    int failed_at = 0;
+#pragma unroll 1
+    for (int n = 0, tile = grp, t = 0; n <= steps && steps > 0; ++n) {
+      const bool issue = n < steps, decode = issue && t == 0, gate = n > 0;
+      const int slot = tile % kRawStages;
+      const unsigned char* st = ring + slot * PG::kStageBytes + row_at;
+      uint4 d = make_uint4(0u, 0u, 0u, 0u);
+      uint2 sf = make_uint2(0u, 0u);  // the row's block scales
+      if (decode) {
+        if (ok && !mbar_wait(&raw_full[slot], (tile / kRawStages) & 1, kBudget, abort_flag)) {
           if (lane == 0) give_up(3, tile);
-          fine = false;
+          ok = false;
+          failed_at = tile;
         }
-        const unsigned char* st = ring + s * PG::kStageBytes;
-        const bool ok = there && page_id[tile * PG::kTilePages + pp] >= 0;
+        // (a page that is not there leaves what the stage held: its rows' scores are replaced)
+        d = *reinterpret_cast<const uint4*>(st + turn);
+        if (FMT == MDC_FMT_NVFP4) sf = *reinterpret_cast<const uint2*>(st + sf_at);
+        else sf.x = *reinterpret_cast<const uint32_t*>(st + sf_at);
+      }
+      float x[4][16], s4[4] = {0.f, 0.f, 0.f, 0.f};
+      // Heads 16c .. 16c + 15 of the row: x + |x| is exactly 0 or 2x; the weighted sums run as packed fp32 pairs.
+      const int done_tile = t == 0 ? tile - G : tile, done_t = t == 0 ? T - 1 : t - 1;   // of step n - 1
+      auto gate_heads = [&](int c, const float (&v)[16]) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) d[k][j] = ok ? *reinterpret_cast<const uint4*>(st + code_at[j]) : make_uint4(0u, 0u, 0u, 0u);
-        raw_sf[k] = make_uint2(0u, 0u);
-        if (ok) {
-          if (FMT == MDC_FMT_NVFP4) raw_sf[k] = *reinterpret_cast<const uint2*>(st + sf_at);
-          else raw_sf[k].x = *reinterpret_cast<const uint32_t*>(st + sf_at);
+        for (int i = 0; i < 4; ++i) {
+          const float4 w = reinterpret_cast<const float4*>(wsc + done_t * kIdxHeads)[4 * c + i];
+          ffma2(s4[0], s4[1], v[4 * i] + fabsf(v[4 * i]), v[4 * i + 1] + fabsf(v[4 * i + 1]), w.x, w.y);
+          ffma2(s4[2], s4[3], v[4 * i + 2] + fabsf(v[4 * i + 2]), v[4 * i + 3] + fabsf(v[4 * i + 3]), w.z, w.w);
+        }
+      };
+      if (gate) {
+        if (ok && !mbar_wait(&mma_done[grp], (n - 1) & 1, kBudget, abort_flag)) {
+          if (lane == 0) give_up(5, tile);
+          ok = false;
+          failed_at = tile;
         }
       }
-      if (!__all_sync(0xffffffffu, fine)) break;
-      // the A pair is free once the MMAs of its previous user, kAPairs pairs ago, are done
-      const int prev = t0 - kASt;
-      if (prev >= 0 && !stages_done(prev, true)) {
-        if (lane == 0) give_up(4, t0);
-        break;
-      }
-      umma::fence_after_sync();
-      // the raw stages are in registers: hand them back to the copy warp
       __syncwarp();
-      mbar_arrive_if(&raw_empty[t0 % kRawStages], lane == 0);
-      mbar_arrive_if(&raw_empty[(t0 + 1) % kRawStages], lane == 0 && two);
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        if (k == 1 && !two) break;
-#pragma unroll
+      umma::fence_after_sync();
+      umma::tmem_ld16_f(t_acc + t_lane, x[0]);   // on its way while the new stage is decoded
+      umma::tmem_ld16_f(t_acc + t_lane + 16, x[1]);
+      if (decode) {
+        // Four copies of this do not stay in a scheduler's instruction cache beside the rest of the step.  In the persistent
+        // kernel that costs more than the loop (step of 8 x 131072 84.7 us unrolled, 79.1 rolled); alone it does not (36.0
+        // against 37.8 for 32 x 32768 tokens).
+        constexpr int kUnroll = ALONE ? 4 : 1;
+#pragma unroll kUnroll
         for (int j = 0; j < 4; ++j) {  // 16-byte chunk j = 32 dims = 16 columns
+          const uint4 following = *reinterpret_cast<const uint4*>(st + (((16 * j + 16) & 48) ^ turn));
           uint32_t s_lo, s_hi;  // fp16x2 block scale of dims 0-15 and 16-31 of the chunk
-          if (FMT == MDC_FMT_NVFP4) {
-            const uint32_t sf2 = (j & 2 ? raw_sf[k].y : raw_sf[k].x) >> (16 * (j & 1));  // scale bytes 2j, 2j+1
-            const uint32_t x = e4m3x2_to_f16x2(static_cast<uint16_t>(sf2 & 0xffff));
-            s_lo = bcast_lo(x);
-            s_hi = bcast_hi(x);
+          if (FMT == MDC_FMT_NVFP4) {   // scale bytes 2j, 2j + 1
+            const uint32_t two = e4m3x2_to_f16x2(static_cast<uint16_t>(sf.x & 0xffff));
+            s_lo = bcast_lo(two);
+            s_hi = bcast_hi(two);
+            sf.x = __funnelshift_r(sf.x, sf.y, 16);
+            sf.y >>= 16;
           } else {
-            s_lo = s_hi = ue8m0_to_f16x2((raw_sf[k].x >> (8 * j)) & 0xff);
+            s_lo = s_hi = ue8m0_to_f16x2(sf.x & 0xff);
+            sf.x >>= 8;
           }
-          const uint32_t w4[4] = {d[k][j].x, d[k][j].y, d[k][j].z, d[k][j].w};
+          const uint32_t w4[4] = {d.x, d.y, d.z, d.w};
           uint32_t out[16];
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
@@ -1452,79 +1410,48 @@ __device__ __forceinline__ int logits_tile(const mdc_logits_params& p, const CUt
 #pragma unroll
             for (int i = 0; i < 4; ++i) out[4 * q4 + i] = hmul2_u32(e[i], q4 < 2 ? s_lo : s_hi);
           }
-          umma::tmem_st16(t_row + ((t0 + k) % kASt) * 64 + 16 * j, out);
+          umma::tmem_st16(t_a + t_lane + 16 * j, out);
+          d = following;
         }
       }
-      // publish the pair as soon as the stores have landed: the tensor core works on it while
-      // this group decodes its next pair
-      umma::wait_st();
-      umma::fence_before_sync();
-      __syncwarp();
-      red_release_cta_shared_inc_if(&a_cnt[pair % kAPairs], lane == 0);
-    }
-  } else {
-    // ---------------- gate warps: thread = token row
-    const int q = (warp - kGateWarp0) & 3, gg = (warp - kGateWarp0) >> 2;
-    const uint32_t t_base = tmem + (static_cast<uint32_t>(q * 32) << 16) + kAccBase;
-    auto emit = [&](int tile, int t, float score) {
-      const int local = tile * kTileTok + q * 32 + lane;  // position inside the chunk
-      if (local < n_pages * PAGE) {
-        const float val = page_id[local / PAGE] >= 0 ? score : neg_inf;
-        if (as_keys) {   // 0 = not a candidate
-          const uint32_t key = blk0 * PAGE + local < limit ? max(sortable_u32(val), 1u) : 0u;
-          reinterpret_cast<uint32_t*>(scores)[t * chunk_tokens + local] = key;
-          if (key) atomicAdd(&hs[t * kThrBins + (key >> kThrShift)], 1u);
-        } else if (fused) scores[t * chunk_tokens + local] = val;
-        else p.logits[(static_cast<int64_t>(b) * T + t) * p.logits_stride + static_cast<int64_t>(blk0) * PAGE + local] = val;
+      // half of the heads while the stores land and the other half is on its way
+      umma::wait_ld();
+      umma::tmem_ld16_f(t_acc + t_lane + 32, x[2]);
+      umma::tmem_ld16_f(t_acc + t_lane + 48, x[3]);
+      if (gate) {
+        gate_heads(0, x[0]);
+        gate_heads(1, x[1]);
       }
-    };
-    constexpr int kStep = kAccPairs ? 2 : 1;   // stages per hand-off; group gg takes the hand-offs gg, gg + GG, ...
-    for (int t0 = gg * kStep; t0 < n_tiles; t0 += GG * kStep) {
-      const bool two = kAccPairs && t0 + 1 < n_tiles;
-      if (!stages_done(t0, two)) {
-        if (lane == 0) give_up(5, t0);
-        break;
-      }
-      umma::fence_after_sync();
-      // two accumulator rows: of the pair's two stages (q_len 1), or of the stage's two query tokens
-      const uint32_t at[2] = {t_base + (t0 % kAccSt) * N,
-                              kAccPairs ? t_base + ((t0 + 1) % kAccSt) * N : t_base + (t0 % kAccSt) * N + kIdxHeads};
-      float sum[2][4], x[2][2][16];
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        sum[r][0] = sum[r][1] = sum[r][2] = sum[r][3] = 0.f;
-        umma::tmem_ld16_f(at[r], x[0][r]);
-      }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {   // 16 heads at a time, the next 16 on their way
-        umma::wait_ld();
-        if (c < 3) {
-#pragma unroll
-          for (int r = 0; r < 2; ++r) umma::tmem_ld16_f(at[r] + 16 * (c + 1), x[(c + 1) & 1][r]);
-        } else {   // the rows are in registers: the accumulators can be overwritten
-          umma::fence_before_sync();
-          __syncwarp();
-          red_release_cta_shared_inc_if(&acc_cnt[(t0 / kStep) & 1], lane == 0);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float4 w = reinterpret_cast<const float4*>(wsc)[4 * c + i];
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            if (!kAccPairs && r == 1) w = reinterpret_cast<const float4*>(wsc + kIdxHeads)[4 * c + i];
-            const float* v = x[c & 1][r] + 4 * i;
-            // x + |x| is exactly 0 or 2x; the weighted sums run as packed fp32 pairs
-            ffma2(sum[r][0], sum[r][1], v[0] + fabsf(v[0]), v[1] + fabsf(v[1]), w.x, w.y);
-            ffma2(sum[r][2], sum[r][3], v[2] + fabsf(v[2]), v[3] + fabsf(v[3]), w.z, w.w);
+      umma::wait_ld();
+      if (issue) {
+        umma::wait_st();
+        umma::fence_before_sync();
+        asm volatile("bar.sync %0, 128;" ::"r"(4 + grp) : "memory");   // A is complete, the accumulator and the raw stage are read
+        if (quad == 0) {
+          umma::fence_after_sync();
+          if (umma::elect_one()) {
+            umma::mma_f16_ts_x8(t_acc, t_a, umma::smem_desc_sw128(qb_u + t * (kIdxHeads * 128)), N * 128, idesc);
+            umma::commit(&mma_done[grp]);
           }
+          __syncwarp();
+        } else if (quad == 1 && decode) {
+          const int next = tile + kRawStages, i = next * PG::kTilePages + lane;
+          refill(ok && next < n_tiles && lane < PG::kTilePages, slot, lane < PG::kTilePages ? lane : 0,
+                 next < n_tiles && lane < PG::kTilePages ? page_id[i] : -1);
+        }
+        if (++t == T) {
+          t = 0;
+          tile += G;
         }
       }
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const float score = (sum[r][0] + sum[r][1]) + (sum[r][2] + sum[r][3]);
-        if (kAccPairs) emit(t0 + r, 0, score);   // (a missing second stage lies behind the last page)
-        else if (r < T) emit(t0, r, score);
-      }
+      if (!gate) continue;
+      gate_heads(2, x[2]);
+      gate_heads(3, x[3]);
+      emit(done_tile * kTileTok + row, done_t, (s4[0] + s4[1]) + (s4[2] + s4[3]));
+    }
+    if (!ok) {   // the group's copies that are still on their way into the ring (bounded, without the block's flag)
+      for (int i = failed_at; i < min(failed_at + kRawStages, n_tiles); i += G)
+        mbar_wait(&raw_full[i % kRawStages], (i / kRawStages) & 1, 1ll << 24);
     }
   }
 
@@ -1533,9 +1460,29 @@ __device__ __forceinline__ int logits_tile(const mdc_logits_params& p, const CUt
   __syncthreads();
   umma::fence_after_sync();
   const bool failed = *abort_flag != 0;
-  if (warp == kIssueWarp) umma::tmem_dealloc(tmem, kTmemCols);
-  if (warp == kCopyWarp && lane < 2 * kRawStages + kAStages) mbar_inval(raw_full + lane);   // the memory is reused by the block's next task
-  const int n_local = n_pages * PAGE, base_pos = blk0 * PAGE;
+  if (warp == kTmemWarp) umma::tmem_dealloc(tmem, kTmemCols);
+  if (warp == kCopyWarp && lane < kRawStages + G) mbar_inval(raw_full + lane);   // the memory is reused by the block's next task
+  return failed ? ~n_pages : n_pages;
+}
+// The tile: the scores, then what becomes of them.  All threads of the block call it.
+// Returns, to the worker threads alike, the entries of the (last) candidate list, or -1 when the row has been published or
+// nothing was written.
+template <int FMT, int PAGE, int T, bool ALONE, bool ROWK = false, bool THR = false>
+__device__ __forceinline__ int logits_tile(const mdc_logits_params& p, const CUtensorMap* pages, int b, int chunk, unsigned char* smem,
+                                           const RowThreshold* rt = nullptr) {
+  using PG = IdxPage<FMT, PAGE>;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int streamed = logits_stream<FMT, PAGE, T, ALONE, ROWK, THR>(p, pages, b, chunk, smem,
+                                                                     THR ? rt->hist_next + static_cast<int64_t>(b) * kThrBins : nullptr);
+  const bool failed = streamed < 0, row_mode = ROWK && p.row_v != nullptr, fused = p.cand_v != nullptr || row_mode;
+  const int n_pages = failed ? ~streamed : streamed, chunk_tokens = p.blocks_per_chunk * PAGE;
+  const bool as_keys = logits_keeps_keys<FMT, PAGE, T, ALONE, THR>(fused, chunk_tokens);
+  const LogitsSmem L = logits_smem_layout<FMT, PAGE>(T, chunk_tokens, fused, as_keys);
+  uint32_t* hs = reinterpret_cast<uint32_t*>(smem + L.hist);
+  unsigned char* ring = smem + L.ring;
+  SelectScratch& sel = *reinterpret_cast<SelectScratch*>(smem + L.sel);
+  float* scores = reinterpret_cast<float*>(smem + L.scores);
+  const int n_local = n_pages * PAGE, base_pos = chunk * chunk_tokens;
   uint32_t* keys0 = reinterpret_cast<uint32_t*>(scores);
   auto put = [&](int t, int pos, int slot) {   // entry `slot` of query token t's list (keys kept as keys)
     const int64_t at = ((static_cast<int64_t>(b) * T + t) * p.n_chunks + chunk) * p.top_k + slot;
@@ -1543,12 +1490,12 @@ __device__ __forceinline__ int logits_tile(const mdc_logits_params& p, const CUt
     p.cand_v[at] = __uint_as_float((kv & 0x80000000u) ? (kv ^ 0x80000000u) : ~kv);
     p.cand_i[at] = (base_pos + pos) * p.id_mul + p.id_add;
   };
-  int32_t* selected = reinterpret_cast<int32_t*>(misc) + 12;       // [T] entries of a token's list, -1: to be selected by a search
-  const bool by_hist = kAlone && as_keys && !(ROWK && row_mode) && !failed;
-  if constexpr (kAlone) {
+  int32_t* selected = reinterpret_cast<int32_t*>(smem + L.misc) + 12;       // [T] entries of a token's list, -1: to be selected by a search
+  const bool by_hist = ALONE && as_keys && !(ROWK && row_mode) && !failed;
+  if constexpr (ALONE) {
     if (by_hist) {
-      // one query token per group of eight warps (the gate warps take the second)
-      static_assert(T == 1 || DG + GG >= 4, "a second group of eight warps");
+      // one query token per group of eight warps
+      static_assert(T == 1 || kLogitsThreads >= 2 * kBlockThreads, "a second group of eight warps");
       HistSelectSmem* hsm = reinterpret_cast<HistSelectSmem*>(ring);   // (the raw ring is idle by now)
       if (warp < kWarps) {
         const int n = hist_select_emit<1>(keys0, n_local, p.top_k, hs, hsm[0], tid, [&](int pos, int slot) { put(0, pos, slot); });
@@ -1576,10 +1523,11 @@ __device__ __forceinline__ int logits_tile(const mdc_logits_params& p, const CUt
     for (int t = 0; t < T; ++t) {
       uint32_t* keys = keys0 + t * chunk_tokens;
       auto emit = [&](int pos, int slot) { put(t, pos, slot); };
-      if (!kAlone && rt) {
+      if constexpr (THR) {
         n = chunk_emit_above_row_threshold(*rt, p.status, b, chunk, p.n_chunks, keys, n_local, base_pos, p.top_k, sel, hs, ring, emit,
                                            p.id_mul, p.id_add);
       } else if (!by_hist) {
+        const int limit = max(0, (p.seq_lens ? p.seq_lens[b] : p.max_pages * PAGE) - p.window_exclude);
         n = fused_chunk_select(scores + t * chunk_tokens, keys, n_local, base_pos, limit, p.top_k, sel, emit);
       } else {
         n = selected[t];

@@ -81,12 +81,6 @@ __host__ __device__ constexpr uint32_t idesc_mla(bool fp8, int M, int N, bool b_
   return (1u << 4) | (fp8 ? 0u : (1u << 7) | (1u << 10)) | (b_mn ? (1u << 16) : 0u) | (static_cast<uint32_t>(N >> 3) << 17) |
          (static_cast<uint32_t>(M >> 4) << 24);
 }
-__device__ inline void tmem_ld32_f(uint32_t taddr, float (&v)[32]) {
-  uint32_t u[32];
-  tmem_ld32(taddr, u);
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(u[i]);
-}
 }  // namespace umma
 
 __device__ inline float ex2_approx(float x) {

@@ -49,6 +49,19 @@ __device__ inline void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
       : "memory");
 }
 
+__device__ inline void tmem_ld32_f(uint32_t taddr, float (&v)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,"
+      "%30,%31}, [%32];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]),
+        "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]),
+        "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]),
+        "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+      : "r"(taddr)
+      : "memory");
+}
+
 __device__ inline void tmem_ld16_f(uint32_t taddr, float (&v)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -114,34 +127,41 @@ __device__ inline void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
         : "memory");
   }
 }
-// One 128-token stage of the indexer: eight K=16 steps into one accumulator,
-// A = 64 consecutive tensor-memory columns (8 per step), B = eight prepared
-// shared-memory descriptors.  A single asm block keeps the issuing thread's
-// instruction count at the minimum (two predicates, then eight MMAs).
-__device__ inline void mma_f16_ts_x8(uint32_t d_tmem, uint32_t a_tmem, const uint64_t (&b)[8], uint32_t idesc) {
+// One 128-token stage of the indexer: eight K=16 steps into one accumulator, A = 64 consecutive tensor-memory columns
+// (8 per step), B = rows of 2 x 128 bytes in shared memory: two 128-byte-swizzled halves `half_bytes` apart, 32 bytes of
+// each row per step.  A single asm block, so that the issuing thread holds one descriptor at a time.
+__device__ inline void mma_f16_ts_x8(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t half_bytes, uint32_t idesc) {
   asm volatile(
       "{\n"
       " .reg .pred pf, pt;\n"
-      " .reg .b32 a1, a2, a3, a4, a5, a6, a7;\n"
+      " .reg .b32 a;\n"
+      " .reg .b64 b, h;\n"
       " setp.ne.b32 pf, 0, 0;\n"
       " setp.eq.b32 pt, 0, 0;\n"
-      " add.u32 a1, %1, 8;\n"
-      " add.u32 a2, %1, 16;\n"
-      " add.u32 a3, %1, 24;\n"
-      " add.u32 a4, %1, 32;\n"
-      " add.u32 a5, %1, 40;\n"
-      " add.u32 a6, %1, 48;\n"
-      " add.u32 a7, %1, 56;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %3, %2, pf;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], %4, %2, pt;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], %5, %2, pt;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], %6, %2, pt;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], [a4], %7, %2, pt;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], [a5], %8, %2, pt;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], [a6], %9, %2, pt;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], [a7], %10, %2, pt;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, pf;\n"
+      " add.u32 a, %1, 8;\n"
+      " add.u64 b, %2, 2;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, pt;\n"
+      " add.u32 a, %1, 16;\n"
+      " add.u64 b, %2, 4;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, pt;\n"
+      " add.u32 a, %1, 24;\n"
+      " add.u64 b, %2, 6;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, pt;\n"
+      " add.u64 h, %2, %4;\n"
+      " add.u32 a, %1, 32;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [a], h, %3, pt;\n"
+      " add.u32 a, %1, 40;\n"
+      " add.u64 b, h, 2;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, pt;\n"
+      " add.u32 a, %1, 48;\n"
+      " add.u64 b, h, 4;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, pt;\n"
+      " add.u32 a, %1, 56;\n"
+      " add.u64 b, h, 6;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, pt;\n"
       "}" ::"r"(d_tmem),
-      "r"(a_tmem), "r"(idesc), "l"(b[0]), "l"(b[1]), "l"(b[2]), "l"(b[3]), "l"(b[4]), "l"(b[5]), "l"(b[6]), "l"(b[7])
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "l"(static_cast<uint64_t>(half_bytes >> 4))
       : "memory");
 }
 // D[tmem] (+)= A[smem] * B[smem]^T

@@ -77,6 +77,29 @@ def test_logits_vs_oracle(fmt, P, T, q_fp4, B, S, bpc):
     assert torch.allclose(got, ref, rtol=1e-3, atol=1e-4), (got - ref).abs().max()
 
 
+@pytest.mark.parametrize("fmt,P,T,q_fp4", [("nvfp4", 64, 1, False), ("nvfp4", 64, 2, False), ("mxfp4", 128, 1, True)])
+@pytest.mark.parametrize("stages", [1, 3, 4, 5, 8, 9, 12, 13, 17])
+def test_logits_stages_of_the_groups(fmt, P, T, q_fp4, stages):
+    """One chunk of fewer and more stages than the four groups and the eight ring slots hold, the last one half full
+    (64-token pages); the second sequence's middle page is not usable: -inf for its tokens, the rest unaffected."""
+    from mega_dsa_cp_b200.tiles.logits import run_fp4_paged_mqa_logits
+
+    pages = stages * (128 // P) - (P == 64)
+    case = indexer_case(2, pages * P, P, fmt, q_len=T, q_fp4=q_fp4, seed=stages, pool_pages=2 * pages + 3)
+    ref = _oracle_logits(case).view(2, T, pages, P)
+    bad = pages // 2
+    case["bt"][1, bad] = -1
+    status = torch.zeros(8, dtype=torch.int32, device=DEV)
+    got = torch.full((2 * T, pages * P), float("nan"), device=DEV)
+    run_fp4_paged_mqa_logits(case["fused"].to(DEV), case["q"].to(DEV), None if case["q_sf"] is None else case["q_sf"].to(DEV),
+                             case["w"].to(DEV), case["bt"].to(DEV), got, pages, fmt=fmt, page_tokens=P, status=status)
+    got = got.cpu().view(2, T, pages, P)
+    assert status[0].item() != 0   # the page is reported
+    assert (got[1, :, bad] == float("-inf")).all()
+    got[1, :, bad] = ref[1, :, bad]
+    assert torch.allclose(got, ref, rtol=1e-3, atol=1e-4), (got - ref).abs().max()   # test_logits_vs_oracle's bound
+
+
 @pytest.mark.parametrize("fmt,P,T,K,bpc,S,seq,wex", [
     ("mxfp4", 128, 2, 512, 32, 8192, 8192, 128),   # the reference's fused test
     ("mxfp4", 128, 2, 1024, 32, 8192, 8000, 128),
