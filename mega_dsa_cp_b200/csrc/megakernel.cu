@@ -581,7 +581,7 @@ __device__ __forceinline__ void op_attn_umma(const mdc_mega_params& p, int b, in
                                           unsigned char* smem) {
   const AttnTarget t = attn_target(p, b, split, phase);
   const mdc_sparse_mla_params mp = attn_params(p, b, phase);
-  mla_umma_tile<DQK>(mp, b, hbv >> 2, hbv & 3, t.split, t.ns, smem, t.slot, t.lse_row, true);
+  mla_umma_tile<DQK, false, false>(mp, b, hbv >> 2, hbv & 3, t.split, t.ns, smem, t.slot, t.lse_row, true, p.layer.cp > 1);
 }
 template <int DQK>
 __device__ __noinline__ void op_attn_umma_call(const mdc_mega_params& p, int b, int hbv, int split, unsigned long long phase,

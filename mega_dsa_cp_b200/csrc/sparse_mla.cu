@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(kMuThreads, 1) mla_umma_kernel(const __grid_co
   wait_for_predecessor();
   let_successor_start();
   const int hb = blockIdx.y >> 2, dq = blockIdx.y & 3;
-  mla_umma_tile<DQK, FP8>(p, blockIdx.z, hb, dq, blockIdx.x, gridDim.x, smem);
+  mla_umma_tile<DQK, FP8, true>(p, blockIdx.z, hb, dq, blockIdx.x, gridDim.x, smem);
 }
 
 template <int DQK, bool FP8>

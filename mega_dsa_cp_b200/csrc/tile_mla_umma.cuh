@@ -155,10 +155,12 @@ __device__ inline uint32_t mla_umma_gather_rows(const mdc_sparse_mla_params& p, 
 // split / n_splits = slice of the slot range.  o_row / lse_row, when given,
 // replace p.o / p.lse for this row (they point at the row's (H, d_v) block and
 // (H,) vector, possibly in a peer GPU's memory); with to_row a split's partial goes there too
-// instead of the split workspace.  All kMuThreads threads call it.
-template <int DQK, bool FP8 = false>
-__device__ void mla_umma_tile(const mdc_sparse_mla_params& p, int r, int hb, int dq, int split, int n_splits,
-                              unsigned char* smem, void* o_row = nullptr, float* lse_row = nullptr, bool to_row = false) {
+// instead of the split workspace.  All threads of the block call it.
+// ALONE: the stand-alone kernel.
+template <int DQK, bool FP8, bool ALONE>
+__device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, int r, int hb, int dq, int split, int n_splits,
+                              unsigned char* smem, void* o_row = nullptr, float* lse_row = nullptr, bool to_row = false,
+                              bool remote = false) {
   using SM = MlaUmmaSmem<DQK, FP8>;
   constexpr int S = SM::kStages, ESZ = FP8 ? 1 : 2, ROWB = SM::kRowBytes;
   constexpr uint32_t kQCols = ROWB / 4, kOCol = kQCols, kSCol = kOCol + kMuDv, kPCol = kSCol + kMuTile;
@@ -166,6 +168,9 @@ __device__ void mla_umma_tile(const mdc_sparse_mla_params& p, int r, int hb, int
   static_assert(S >= 3 && SM::kPanels * kMuHeads * 128 <= (S - 1) * SM::kStageBytes,
                 "two tiles are held while the next is gathered, and the staged query must fit the KV ring behind its first stage");
   constexpr long long kBudget = 1ll << 31;
+  // Warps of a lane quadrant that move the query into tensor memory: the softmax warp and, stand-alone, two gather warps (32 rows x
+  // 2048 slots 49.0 -> 48.1 us; inside the persistent kernel the three of them gained nothing).
+  constexpr int kMovers = ALONE ? 3 : 1;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned char* kst = smem + SM::kK;
   unsigned char* qst = kst + SM::kStageBytes;   // the query rows are staged in stages 1.. while tile 0 lands in stage 0
@@ -203,7 +208,7 @@ __device__ void mla_umma_tile(const mdc_sparse_mla_params& p, int r, int hb, int
     mbar_init(s_ready, 1);
     mbar_init(s_taken, 4);
     mbar_init(p_ready, 4);
-    mbar_init(q_ready, 4);
+    mbar_init(q_ready, 4 * kMovers);
     mbar_init(o_final, 1);
     mbar_init(qs_ready, kMuGatherWarps);
     misc[1] = 0;
@@ -219,32 +224,36 @@ __device__ void mla_umma_tile(const mdc_sparse_mla_params& p, int r, int hb, int
     *abort_flag = 1;
   };
 
+  // Query rows -> tensor memory (16 columns per store), from the copy the gather warps staged
+  // in the (still empty) stages 1.. of the KV ring as panels of 128 rows x 128 bytes, 128-byte swizzle.  Mover
+  // `m` of its lane quadrant (a warp's number % 4) takes every kMovers-th 16 columns.
+  auto query_to_tmem = [&](int m) {
+    if (!mbar_wait(qs_ready, 0, kBudget, abort_flag) && lane == 0) give_up(7, 0);
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t t_row = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+#pragma unroll 2
+    for (int j = m; j < static_cast<int>(kQCols) / 16; j += kMovers) {
+      uint32_t v[16];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int ch = 4 * j + u;
+        const uint4 x = *reinterpret_cast<const uint4*>(qst + (ch >> 3) * (kMuHeads * 128) + row * 128 +
+                                                        (((ch & 7) ^ (row & 7)) << 4));
+        v[4 * u] = x.x; v[4 * u + 1] = x.y; v[4 * u + 2] = x.z; v[4 * u + 3] = x.w;
+      }
+      umma::tmem_st16(t_row + 16 * j, v);
+    }
+    umma::wait_st();
+    umma::fence_before_sync();
+    __syncwarp();
+    mbar_arrive_if(q_ready, lane == 0);
+  };
+
   if (warp < 4) {
     // ---------------- softmax warps: thread = head
     const int h = hb * kMuHeads + warp * 32 + lane;
     const uint32_t t_lane = tmem + (static_cast<uint32_t>(warp * 32) << 16);
-    {  // Q row -> tensor memory (16 columns per store), from the copy the gather warps staged
-      // in the (still empty) stages 1.. of the KV ring as panels of 128 rows x 128 bytes, 128-byte swizzle
-      bool okq = mbar_wait(qs_ready, 0, kBudget, abort_flag);
-      if (!okq && lane == 0) give_up(7, 0);
-      const int row = warp * 32 + lane;
-#pragma unroll 2
-      for (int j = 0; j < static_cast<int>(kQCols) / 16; ++j) {
-        uint32_t v[16];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int ch = 4 * j + u;
-          const uint4 x = *reinterpret_cast<const uint4*>(qst + (ch >> 3) * (kMuHeads * 128) + row * 128 +
-                                                          (((ch & 7) ^ (row & 7)) << 4));
-          v[4 * u] = x.x; v[4 * u + 1] = x.y; v[4 * u + 2] = x.z; v[4 * u + 3] = x.w;
-        }
-        umma::tmem_st16(t_lane + 16 * j, v);
-      }
-      umma::wait_st();
-      umma::fence_before_sync();
-      __syncwarp();
-      mbar_arrive_if(q_ready, lane == 0);
-    }
+    query_to_tmem(0);
     float m_used = neg_inf, l = 0.f;
     if (p.attn_sink && split == 0) {
       const float sk = p.attn_sink[h];
@@ -381,11 +390,13 @@ __device__ void mla_umma_tile(const mdc_sparse_mla_params& p, int r, int hb, int
         }
       }
       const int col0 = dq * kMuDv;
-      // A bf16 row that goes to o_row (the owner's inbox, possibly on a peer GPU) is staged in shared
-      // memory (the KV ring is idle now) and leaves as ONE 256-byte bulk copy per head: sixteen
-      // 16-byte stores per thread over NVLink take an order of magnitude longer.
-      const bool bulk_out = direct && o_row != nullptr && p.out_dtype != MDC_DT_F32;
-      unsigned char* stage_row = kst + (warp * 32 + lane) * (kMuDv * 2);
+      // A bf16 row that goes to o_row (the owner's inbox) is staged in shared memory (the KV ring is idle now).  To a peer GPU
+      // it leaves as ONE 256-byte bulk copy per head: sixteen 16-byte stores per thread over NVLink take an order of magnitude
+      // longer.  On this GPU the warp stores its 32 rows, two per instruction (step of 1 x 4096 tokens 42.9 -> 41.7 us,
+      // 8 x 131072 79.2 -> 78.1: the copies' completion had to be waited for before the notify).
+      const bool stage_out = direct && o_row != nullptr && p.out_dtype != MDC_DT_F32;
+      constexpr int kPitch = kMuDv * 2 + 16;   // (the 16 bytes keep a warp's stores off one bank)
+      unsigned char* stage_row = kst + (warp * 32 + lane) * kPitch;
 #pragma unroll 1
       for (int cb = 0; cb < kMuDv / 32; ++cb) {
         float o[32];
@@ -399,7 +410,7 @@ __device__ void mla_umma_tile(const mdc_sparse_mla_params& p, int r, int hb, int
 #pragma unroll
         for (int j = 0; j < 32; ++j) o[j] *= inv;
         const int col = col0 + 32 * cb;
-        if (bulk_out) {
+        if (stage_out) {
           uint4* dst = reinterpret_cast<uint4*>(stage_row + 64 * cb);
 #pragma unroll
           for (int j = 0; j < 4; ++j)
@@ -426,7 +437,16 @@ __device__ void mla_umma_tile(const mdc_sparse_mla_params& p, int r, int hb, int
                                 pack_bf16x2(o[8 * j + 4], o[8 * j + 5]), pack_bf16x2(o[8 * j + 6], o[8 * j + 7]));
         }
       }
-      if (bulk_out) {
+      if (stage_out && !remote) {
+        __syncwarp();
+        unsigned char* to = static_cast<unsigned char*>(o_row) + (static_cast<int64_t>(h - lane) * kMlaDv + col0) * 2;
+        const unsigned char* from = kst + warp * 32 * kPitch;
+#pragma unroll 4
+        for (int i = lane; i < 32 * (kMuDv / 8); i += 32) {   // row i / 16, 16 bytes each
+          const int rr = i / (kMuDv / 8), ch = i % (kMuDv / 8);
+          *reinterpret_cast<uint4*>(to + rr * (kMlaDv * 2) + ch * 16) = *reinterpret_cast<const uint4*>(from + rr * kPitch + ch * 16);
+        }
+      } else if (stage_out) {
         fence_proxy_async_smem();  // the copy engine reads the staged row through the async proxy
         bulk_s2g(static_cast<__nv_bfloat16*>(o_row) + static_cast<int64_t>(h) * kMlaDv + col0, stage_row, kMuDv * 2);
         bulk_commit();
@@ -473,7 +493,8 @@ __device__ void mla_umma_tile(const mdc_sparse_mla_params& p, int r, int hb, int
     {
       __syncwarp();
       mbar_arrive_if(qs_ready, lane == 0);
-      // stages 1.. are free for KV tiles once the softmax warps have moved the rows into tensor memory
+      if constexpr (ALONE) query_to_tmem(warp / 4);
+      // stages 1.. are free for KV tiles once all of them have moved their share
       if (!mbar_wait(q_ready, 0, kBudget, abort_flag)) {
         if (lane == 0) give_up(8, 0);
         ok = false;
