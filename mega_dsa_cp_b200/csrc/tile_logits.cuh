@@ -603,11 +603,12 @@ static __device__ __noinline__ bool chunk_publish_row_one_rank(const RowThreshol
   const RowOneRank& one = x.one;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lt = (1u << lane) - 1u;
+  uint32_t off = 0u;   // (thread 0) the chunk's place in the row's list: a round trip to L2 under the search for the survivors
   if (tid == 0) {
     sm.n_s = sm.n_above = sm.n_mine = 0;
     sm.n_few = sm.need_eq = 0;
     sm.sums[0] = sm.sums[1] = sm.sums[2] = sm.sums[3] = 0;
-    sm.off = bin && n_und ? static_cast<int>(atomicAdd(one.count, n_und)) : 0;
+    if (bin && n_und) off = atomicAdd(one.count, n_und);
     if (chunk == 0) *one.count_next = 0u;
   }
   sync_workers();
@@ -641,6 +642,7 @@ static __device__ __noinline__ bool chunk_publish_row_one_rank(const RowThreshol
       at += __popc(m[j]);
     }
   }
+  if (tid == 0) sm.off = static_cast<int>(off);
   sync_workers();
   const int n_s = min(sm.n_s, kSurvCap);
   // ---- those inside the boundary bin -> the row's list
