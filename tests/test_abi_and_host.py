@@ -457,3 +457,16 @@ def test_ctypes_mirrors_match_the_header_layout(tmp_path):
         assert int(got[cname]) == C.sizeof(mirror), (cname, got[cname], C.sizeof(mirror))
         for fname, _ in mirror._fields_:
             assert int(got[f"{cname}.{fname}"]) == getattr(mirror, fname).offset, (cname, fname)
+
+
+def test_lse_merge_tasks_stay_within_a_wave_and_cover_the_heads():
+    from mega_dsa_cp_b200.layer import build_layer_dag, lse_groups_for
+
+    for owned in (1, 8, 14, 15, 18, 19, 37, 38, 74, 200):
+        g = lse_groups_for(owned, 148)
+        assert g == 2 or owned * g <= 148
+        per = -(-128 // g)
+        assert sorted(h for q in range(g) for h in range(q * per, min(128, (q + 1) * per))) == list(range(128))
+    tasks, _, ops = build_layer_dag(3, 4, 1, lse_groups=4)
+    from mega_dsa_cp_b200 import _native as N
+    assert [t.coords for t in tasks if ops[t.name] == N.OP_LSE_MERGE] == [(b, q, 4) for b in range(3) for q in range(4)]
