@@ -4,7 +4,7 @@
 // Cross-rank payload travels by direct stores / bulk copies into the peers'
 // symmetric arena, followed by a system-scope release notify.
 //
-// Block shape: 16 warps, which leave a thread 128 registers.  Warps 0..7 are the workers every tile is written
+// Block shape: 14 warps (kMegaThreads), which leave a thread 128 registers.  Warps 0..7 are the workers every tile is written
 // for; the indexer, attention and LSE-merge tiles use the others too.
 // Blocks wait on each other, so the grid must be co-resident (<= one block per
 // SM; the launcher checks it).  Every wait has a time budget; a block that
@@ -24,7 +24,6 @@
 
 namespace mdc {
 
-constexpr int kMegaThreads = kLogitsThreads;
 static_assert(kMegaThreads >= kMuThreads, "the block must hold the attention tile's warps (its roles go by warp index; extra warps only join the barriers)");
 constexpr int kStagedWords = 128;  // queue rows up to this length are staged in shared memory
 constexpr int kMegaTileSmem = MlaUmmaSmem<576>::kTotal > MlaSmem<576>::kTotal ? MlaUmmaSmem<576>::kTotal : MlaSmem<576>::kTotal;  // the largest tile
@@ -371,7 +370,7 @@ __device__ __forceinline__ int op_logits(const mdc_mega_params& p, const CUtenso
 
 // The operations of the default layer (NVFP4 pages of 64 tokens, row threshold, bf16 attention over 576 dims, LSE merge) stand
 // in the kernel's body: a call keeps 32 registers from a function, which has to save them.  The other forms are functions, to
-// keep the body short (step of 8 x 131072 with all of them functions 83.3 us, with these three inside 79.1).
+// keep the body short (step of 8 x 131072, four indexer groups, with all of them functions 83.3 us, with these three inside 79.1).
 template <int FMT, int PAGE, bool THR>
 __device__ __noinline__ int op_logits_call(const mdc_mega_params& p, const CUtensorMap* pages, int b, int chunk, unsigned long long phase,
                                            unsigned char* smem) {

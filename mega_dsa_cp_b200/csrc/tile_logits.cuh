@@ -3,13 +3,13 @@
 // writes the fp32 logits row or keeps the chunk's scores in shared memory and
 // emits the exact local top-k.
 //
-// Four groups of four warps take the 128-token stages in turn, each with tensor memory, a slot pair of the raw ring
-// and barriers of its own:
+// Groups of four warps (four stand-alone, three in the persistent kernel) take the 128-token stages in turn, each with
+// tensor memory, a slot pair of the raw ring and barriers of its own:
 //
 //   copy     a page is contiguous in HBM (P x 64 B of packed E2M1, then the page's block scales); one tiled TMA load
 //            per page fills a raw stage in shared memory and swizzles its 64-byte rows on the way (16-byte chunk j of
 //            row r at j ^ (r / 2 % 4)), which is what makes the row loads below bank-conflict free.  The group that
-//            has read a stage loads the stage kRawStages further on into it.
+//            has read a stage loads the stage two of its turns further on into it.
 //   decode   thread i of a group owns token row i: it reads 64 B of codes (four 16-byte loads) and the row's scales,
 //            converts with cvt.f16x2.e2m1x2, multiplies by the block scale (exact in fp16) and stores the row into
 //            TENSOR MEMORY (tcgen05.st) as the A operand.
@@ -30,9 +30,14 @@
 // its own product, both of which have had most of a step to complete.  The form before had two decode groups, two gate
 // groups, two issue warps and a copy warp (one gate group and one issue warp in the persistent kernel), handing stages on
 // in pairs.  32 x 32768 tokens with row top-k 38.9 -> 36.0 us, 37 sequences x 16384 tokens, logits out, 18.0 -> 15.4,
-// two query tokens, 16 x 32768 MXFP4, 32.2 -> 29.0, 3 x 20032 6.4 -> 5.1 (of which the query's loads in flight together
-// 1.0), the persistent kernel's step of 8 x 131072 84.6 -> 79.1.  Three groups, with issue and copy warps: 43.5 for the
+// two query tokens, 16 x 32768 MXFP4, 32.2 -> 28.8, 3 x 20032 6.4 -> 5.1 (of which the query's loads in flight together
+// 1.0), the persistent kernel's step of 8 x 131072 85.5 -> 76.3 with what else changed there.
+// Three groups with issue and copy warps between them: 43.5 for the
 // first of these; the warps of a group taking turns to issue: 37.7.
+//
+// The persistent kernel's blocks have 14 warps: three groups there.  Four, in blocks of 16 warps, need the decode loop rolled,
+// or the step's code does not stay in the instruction cache (step of 8 x 131072 84.7 us unrolled, 78.2 rolled; three
+// groups 79.7 rolled, 76.3 unrolled).
 //
 // Exactness.  K values (E2M1 x scale) are exact in fp16.  Query rows are
 // rescaled per head by a power of two so that the largest element lands in
@@ -65,6 +70,9 @@ constexpr int kRawStages = 8;    // raw page ring: two slots per group
 constexpr int kTmemCols = 512;   // per group 64 columns of accumulator (128 rows x 64 heads) and 64 of decoded A
 constexpr int kFusedRegE = 32;   // fused top-k keeps up to 256 * 32 scores per query token in registers
 constexpr int kLogitsThreads = kLogitsGroups * 128;
+// The persistent kernel: three groups (see above) and six of the stages.
+constexpr int kMegaGroups = 3, kMegaThreads = 448;
+static_assert(kMegaGroups * 128 <= kMegaThreads && kMegaGroups <= kLogitsGroups, "the groups' warps");
 static_assert(kRawStages % kLogitsGroups == 0 && kLogitsGroups * 128 <= kTmemCols, "slots and columns of the groups");
 
 template <int FMT, int PAGE>
@@ -1216,7 +1224,8 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
                                              uint32_t* hist_next) {
   using PG = IdxPage<FMT, PAGE>;
   constexpr int N = T * kIdxHeads;
-  constexpr int G = kLogitsGroups, kThreads = kLogitsThreads;
+  constexpr int G = ALONE ? kLogitsGroups : kMegaGroups, NS = 2 * G;   // groups, raw stages in use
+  constexpr int kThreads = ALONE ? kLogitsThreads : kMegaThreads;
   constexpr int kCopyWarp = kWarps, kTmemWarp = kWarps + 1;   // set-up: the first ring fill and the barriers; tensor memory
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool fused = p.cand_v != nullptr || (ROWK && p.row_v != nullptr);
@@ -1228,7 +1237,7 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
   unsigned char* qb = smem + L.qb;
   unsigned char* ring = smem + L.ring;
   uint64_t* raw_full = reinterpret_cast<uint64_t*>(smem + L.bars);
-  uint64_t* mma_done = raw_full + kRawStages;   // [G]: the group's product is complete
+  uint64_t* mma_done = raw_full + NS;   // [G]: the group's product is complete
   uint32_t* misc = reinterpret_cast<uint32_t*>(smem + L.misc);
   volatile uint32_t* abort_flag = misc + 1;
   int32_t* page_id = reinterpret_cast<int32_t*>(smem + L.page_ok);
@@ -1267,7 +1276,7 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
   };
   if (warp == kCopyWarp) {
     if (lane == 0) {
-      for (int s = 0; s < kRawStages + G; ++s) mbar_init(&raw_full[s], 1);
+      for (int s = 0; s < NS + G; ++s) mbar_init(&raw_full[s], 1);
       for (int i = 1; i < 16; ++i) misc[i] = 0;
       mbar_fence_init();
     }
@@ -1276,7 +1285,7 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
     // (read up to the chunk's end: the load does not wait for the sequence's length)
     int id = lane < table_end ? bt[blk0 + lane] : -1;
     if (lane >= n_pages || id >= p.num_pages) id = -1;
-    refill(lane < min(kRawStages, n_tiles) * PG::kTilePages, lane / PG::kTilePages, lane % PG::kTilePages, id);
+    refill(lane < min(NS, n_tiles) * PG::kTilePages, lane / PG::kTilePages, lane % PG::kTilePages, id);
   } else if (warp < kWarps) {
     logits_stage_query<T>(p, b, qb, wsc);
     fence_proxy_async_smem();  // the tensor core reads the query block through the async proxy
@@ -1341,18 +1350,18 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
     // are computed.  A wait that runs out leaves the loop's barriers in place: every warp of the group walks them all.
     // (The tensor-memory loads stand outside the conditions, the first step's read nothing of use: inside the persistent
     // kernel conditional ones made every function of it spill.)
-    const int steps = n_tiles > grp ? ceil_div(n_tiles - grp, G) * T : 0;
+    const int steps = grp < G && n_tiles > grp ? ceil_div(n_tiles - grp, G) * T : 0;
     bool ok = true;
     int failed_at = 0;
 #pragma unroll 1
     for (int n = 0, tile = grp, t = 0; n <= steps && steps > 0; ++n) {
       const bool issue = n < steps, decode = issue && t == 0, gate = n > 0;
-      const int slot = tile % kRawStages;
+      const int slot = tile % NS;
       const unsigned char* st = ring + slot * PG::kStageBytes + row_at;
       uint4 d = make_uint4(0u, 0u, 0u, 0u);
       uint2 sf = make_uint2(0u, 0u);  // the row's block scales
       if (decode) {
-        if (ok && !mbar_wait(&raw_full[slot], (tile / kRawStages) & 1, kBudget, abort_flag)) {
+        if (ok && !mbar_wait(&raw_full[slot], (tile / NS) & 1, kBudget, abort_flag)) {
           if (lane == 0) give_up(3, tile);
           ok = false;
           failed_at = tile;
@@ -1385,11 +1394,7 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
       umma::tmem_ld16_f(t_acc + t_lane, x[0]);   // on its way while the new stage is decoded
       umma::tmem_ld16_f(t_acc + t_lane + 16, x[1]);
       if (decode) {
-        // Four copies of this do not stay in a scheduler's instruction cache beside the rest of the step.  In the persistent
-        // kernel that costs more than the loop (step of 8 x 131072 84.7 us unrolled, 79.1 rolled); alone it does not (36.0
-        // against 37.8 for 32 x 32768 tokens).
-        constexpr int kUnroll = ALONE ? 4 : 1;
-#pragma unroll kUnroll
+#pragma unroll
         for (int j = 0; j < 4; ++j) {  // 16-byte chunk j = 32 dims = 16 columns
           const uint4 following = *reinterpret_cast<const uint4*>(st + (((16 * j + 16) & 48) ^ turn));
           uint32_t s_lo, s_hi;  // fp16x2 block scale of dims 0-15 and 16-31 of the chunk
@@ -1437,7 +1442,7 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
           }
           __syncwarp();
         } else if (quad == 1 && decode) {
-          const int next = tile + kRawStages, i = next * PG::kTilePages + lane;
+          const int next = tile + NS, i = next * PG::kTilePages + lane;
           refill(ok && next < n_tiles && lane < PG::kTilePages, slot, lane < PG::kTilePages ? lane : 0,
                  next < n_tiles && lane < PG::kTilePages ? page_id[i] : -1);
         }
@@ -1452,8 +1457,8 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
       emit(done_tile * kTileTok + row, done_t, (s4[0] + s4[1]) + (s4[2] + s4[3]));
     }
     if (!ok) {   // the group's copies that are still on their way into the ring (bounded, without the block's flag)
-      for (int i = failed_at; i < min(failed_at + kRawStages, n_tiles); i += G)
-        mbar_wait(&raw_full[i % kRawStages], (i / kRawStages) & 1, 1ll << 24);
+      for (int i = failed_at; i < min(failed_at + NS, n_tiles); i += G)
+        mbar_wait(&raw_full[i % NS], (i / NS) & 1, 1ll << 24);
     }
   }
 
@@ -1463,7 +1468,7 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
   umma::fence_after_sync();
   const bool failed = *abort_flag != 0;
   if (warp == kTmemWarp) umma::tmem_dealloc(tmem, kTmemCols);
-  if (warp == kCopyWarp && lane < kRawStages + G) mbar_inval(raw_full + lane);   // the memory is reused by the block's next task
+  if (warp == kCopyWarp && lane < NS + G) mbar_inval(raw_full + lane);   // the memory is reused by the block's next task
   return failed ? ~n_pages : n_pages;
 }
 // The tile: the scores, then what becomes of them.  All threads of the block call it.
