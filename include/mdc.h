@@ -40,7 +40,7 @@ extern "C" {
 /* device-side status codes (status[0]) */
 #define MDC_DEV_OK 0
 #define MDC_DEV_WAIT_TIMEOUT 1   /* event wait gave up: [2]=event id            */
-#define MDC_DEV_COPY_TIMEOUT 2   /* staged copy never completed: [2]=stage      */
+#define MDC_DEV_COPY_TIMEOUT 2   /* a copy or product never completed: [2]=which wait of the tile, [3]=stage */
 #define MDC_DEV_BAD_INDEX 3      /* page / entry id out of range: [2]=id        */
 #define MDC_DEV_BAD_OP 4         /* unknown task op code: [2]=op                */
 #define MDC_DEV_ABORTED 5        /* left early because another block failed     */
@@ -336,6 +336,11 @@ typedef struct {
   int32_t* status;
 } mdc_pingpong_params;
 int mdc_test_pingpong_launch(const mdc_pingpong_params* p, void* stream);
+
+/* Host arithmetic of the indexer's failure path, for the CPU tests: the stages [first_end[0], first_end[1]) in steps of
+ * `groups` whose copies a group may have on their way when it gives up in front of the product of stage `tile` and query
+ * token t. */
+int mdc_test_stages_on_their_way(int32_t tile, int32_t t, int32_t groups, int32_t n_tiles, int32_t* first_end);
 
 /* task op codes understood by mdc_megakernel_launch */
 #define MDC_OP_NOP 0

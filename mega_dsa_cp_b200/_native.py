@@ -155,7 +155,7 @@ EXPORTS = [
     "mdc_sparse_mla_launch_static_ws",
     "mdc_megakernel_launch", "mdc_megakernel_check", "mdc_megakernel_smem_bytes", "mdc_megakernel_threads",
     "mdc_compress_step_launch", "mdc_compress_finalize_launch", "mdc_hadamard_quant_launch",
-    "mdc_test_pingpong_launch", "mdc_causal_lens_launch",
+    "mdc_test_pingpong_launch", "mdc_test_stages_on_their_way", "mdc_causal_lens_launch",
 ]
 
 

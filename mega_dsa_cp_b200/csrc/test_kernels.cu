@@ -3,6 +3,7 @@
 // whose event is already complete.  Every wait is bounded; a wait that runs out is reported through the
 // status block and ends the kernel.
 #include "events.cuh"
+#include "tile_logits.cuh"
 
 namespace mdc {
 
@@ -52,5 +53,14 @@ extern "C" int mdc_test_pingpong_launch(const mdc_pingpong_params* p, void* stre
   if (p->role == 2 && p->peer != p->events.my_rank) return MDC_ERR_BAD_SHAPE;
   pingpong_kernel<<<p->role == 2 ? 2 : 1, 32, 0, static_cast<cudaStream_t>(stream)>>>(*p);
   MDC_CUDA_OK(cudaGetLastError());
+  return MDC_OK;
+}
+
+extern "C" int mdc_test_stages_on_their_way(int32_t tile, int32_t t, int32_t groups, int32_t n_tiles, int32_t* first_end) {
+  if (!first_end) return MDC_ERR_NULL;
+  if (tile < 0 || t < 0 || groups < 1 || n_tiles < 0) return MDC_ERR_BAD_SHAPE;
+  const mdc::StageRange r = mdc::stages_on_their_way(tile, t, groups, n_tiles);
+  first_end[0] = r.first;
+  first_end[1] = r.end;
   return MDC_OK;
 }

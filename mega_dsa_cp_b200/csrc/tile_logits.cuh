@@ -1215,6 +1215,18 @@ __device__ __forceinline__ bool logits_keeps_keys(bool fused, int chunk_tokens) 
   return ALONE ? fused && logits_as_keys<FMT, PAGE>(T, chunk_tokens) : THR;
 }
 
+// The stages whose copies a group may have on their way when it gives up in front of the product of `tile` and query token
+// t: first, first + groups, ... below end.  (A group's stages are first loaded two at a time; its stage `tile` is handed the
+// copy of tile + 2 * groups once it is decoded, with t = 0.  A stage that has been waited for is not in the range: its
+// barrier may be two phases on, which a wait by parity takes for not complete.)
+struct StageRange {
+  int first, end;
+};
+__host__ __device__ inline StageRange stages_on_their_way(int tile, int t, int groups, int n_tiles) {
+  const int first = t > 0 ? tile + groups : tile;
+  return {first, first + 2 * groups < n_tiles ? first + 2 * groups : n_tiles};
+}
+
 // Scores the chunk.  smem: dynamic shared memory base (1024 B aligned), laid out by logits_smem_layout.  All threads of the
 // block call it.  ALONE: the stand-alone kernels; THR: the persistent kernel with a row threshold, `hist_next`: the row's
 // histogram of the next step, of which this task zeroes its slice.  Returns the chunk's pages, or their complement (< 0) when
@@ -1256,7 +1268,7 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
   const int32_t* bt = p.block_table + static_cast<int64_t>(b) * p.max_pages;
   const int table_end = min(p.blocks_per_chunk, p.max_pages - blk0);   // the chunk's entries of the page table
   int bad_page = 0;
-  constexpr long long kBudget = 1ll << 31;  // clock cycles a role waits before it gives up
+  constexpr long long kBudget = 1ll << 31, kDrain = 1ll << 24;  // clock cycles a role waits before it gives up, and after
 
   // ---------------- prologue.  One warp fills the ring at once; the query, the page table and tensor memory are
   // set up meanwhile.
@@ -1347,25 +1359,23 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
     constexpr uint32_t idesc = umma::idesc_f16(kTileTok, kIdxHeads, 0);
     const uint32_t qb_u = smem_u32(qb);
     // Step n of the group: the product of stage grp + G * (n / T) and query token n % T is issued, the scores of step n - 1
-    // are computed.  A wait that runs out leaves the loop's barriers in place: every warp of the group walks them all.
+    // are computed.  A wait that runs out in any lane ends its warp's steps: it issues and writes nothing more, walks the
+    // barriers that are left (the group's other warps go on until the block's flag ends a wait of theirs, or to the end) and
+    // waits for what it has put on its way.
     // (The tensor-memory loads stand outside the conditions, the first step's read nothing of use: inside the persistent
     // kernel conditional ones made every function of it spill.)
     const int steps = grp < G && n_tiles > grp ? ceil_div(n_tiles - grp, G) * T : 0;
-    bool ok = true;
-    int failed_at = 0;
+    int n = 0, tile = grp, t = 0;
 #pragma unroll 1
-    for (int n = 0, tile = grp, t = 0; n <= steps && steps > 0; ++n) {
+    for (; n <= steps && steps > 0; ++n) {
       const bool issue = n < steps, decode = issue && t == 0, gate = n > 0;
       const int slot = tile % NS;
       const unsigned char* st = ring + slot * PG::kStageBytes + row_at;
       uint4 d = make_uint4(0u, 0u, 0u, 0u);
       uint2 sf = make_uint2(0u, 0u);  // the row's block scales
+      bool there = true, done = true;   // the raw stage; the product
       if (decode) {
-        if (ok && !mbar_wait(&raw_full[slot], (tile / NS) & 1, kBudget, abort_flag)) {
-          if (lane == 0) give_up(3, tile);
-          ok = false;
-          failed_at = tile;
-        }
+        there = mbar_wait(&raw_full[slot], (tile / NS) & 1, kBudget, abort_flag);
         // (a page that is not there leaves what the stage held: its rows' scores are replaced)
         d = *reinterpret_cast<const uint4*>(st + turn);
         if (FMT == MDC_FMT_NVFP4) sf = *reinterpret_cast<const uint2*>(st + sf_at);
@@ -1382,14 +1392,8 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
           ffma2(s4[2], s4[3], v[4 * i + 2] + fabsf(v[4 * i + 2]), v[4 * i + 3] + fabsf(v[4 * i + 3]), w.z, w.w);
         }
       };
-      if (gate) {
-        if (ok && !mbar_wait(&mma_done[grp], (n - 1) & 1, kBudget, abort_flag)) {
-          if (lane == 0) give_up(5, tile);
-          ok = false;
-          failed_at = tile;
-        }
-      }
-      __syncwarp();
+      if (gate && there) done = mbar_wait(&mma_done[grp], (n - 1) & 1, kBudget, abort_flag);
+      const bool go = __all_sync(0xffffffffu, there && done);   // (the lanes may have seen the last poll differently)
       umma::fence_after_sync();
       umma::tmem_ld16_f(t_acc + t_lane, x[0]);   // on its way while the new stage is decoded
       umma::tmem_ld16_f(t_acc + t_lane + 16, x[1]);
@@ -1423,6 +1427,11 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
       }
       // half of the heads while the stores land and the other half is on its way
       umma::wait_ld();
+      if (!go) {
+        const bool all_there = __all_sync(0xffffffffu, there);
+        if (lane == 0) give_up(all_there ? 5 : 3, tile);
+        break;
+      }
       umma::tmem_ld16_f(t_acc + t_lane + 32, x[2]);
       umma::tmem_ld16_f(t_acc + t_lane + 48, x[3]);
       if (gate) {
@@ -1443,7 +1452,7 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
           __syncwarp();
         } else if (quad == 1 && decode) {
           const int next = tile + NS, i = next * PG::kTilePages + lane;
-          refill(ok && next < n_tiles && lane < PG::kTilePages, slot, lane < PG::kTilePages ? lane : 0,
+          refill(next < n_tiles && lane < PG::kTilePages, slot, lane < PG::kTilePages ? lane : 0,
                  next < n_tiles && lane < PG::kTilePages ? page_id[i] : -1);
         }
         if (++t == T) {
@@ -1456,9 +1465,14 @@ __device__ __forceinline__ int logits_stream(const mdc_logits_params& p, const C
       gate_heads(3, x[3]);
       emit(done_tile * kTileTok + row, done_t, (s4[0] + s4[1]) + (s4[2] + s4[3]));
     }
-    if (!ok) {   // the group's copies that are still on their way into the ring (bounded, without the block's flag)
-      for (int i = failed_at; i < min(failed_at + NS, n_tiles); i += G)
-        mbar_wait(&raw_full[i % NS], (i / NS) & 1, 1ll << 24);
+    if (steps > 0 && n <= steps) {   // gave up in step n (alike in the warp's lanes)
+      umma::wait_st();
+      for (int i = n; i < steps; ++i) asm volatile("bar.sync %0, 128;" ::"r"(4 + grp) : "memory");
+      // (bounded, without the block's flag)
+      if (quad == 0 && n > 0) mbar_wait(&mma_done[grp], (n - 1) & 1, kDrain);
+      const StageRange on_way = stages_on_their_way(tile, t, G, n_tiles);
+      if (quad == 1)
+        for (int i = on_way.first; i < on_way.end; i += G) mbar_wait(&raw_full[i % NS], (i / NS) & 1, kDrain);
     }
   }
 

@@ -470,3 +470,28 @@ def test_lse_merge_tasks_stay_within_a_wave_and_cover_the_heads():
     tasks, _, ops = build_layer_dag(3, 4, 1, lse_groups=4)
     from mega_dsa_cp_b200 import _native as N
     assert [t.coords for t in tasks if ops[t.name] == N.OP_LSE_MERGE] == [(b, q, 4) for b in range(3) for q in range(4)]
+
+
+@pytest.mark.parametrize("groups", [3, 4])
+@pytest.mark.parametrize("q_len", [1, 2])
+def test_indexer_group_that_gives_up_waits_for_all_its_copies(groups, q_len):
+    """The order in which an indexer group loads and awaits its stages, walked up to every point at which it can give up:
+    what is loaded and not awaited there is what it waits for before the block leaves, neither less nor more (the barrier
+    of an awaited stage may be two phases on, and a wait for it would not end)."""
+    from mega_dsa_cp_b200 import _native as N
+
+    out = (C.c_int32 * 2)()
+    for n_tiles in range(1, 6 * groups + 2):
+        for grp in range(groups):
+            mine = range(grp, n_tiles, groups)
+            loaded, awaited = {t for t in mine if t < 2 * groups}, set()
+            for tile in mine:
+                for t in range(q_len):
+                    assert N.lib().mdc_test_stages_on_their_way(tile, t, groups, n_tiles, out) == 0
+                    assert set(range(out[0], out[1], groups)) == loaded - awaited, (n_tiles, grp, tile, t)
+                    if t == 0:
+                        awaited.add(tile)
+                        loaded |= {tile + 2 * groups} & set(mine)
+            past = grp + len(mine) * groups   # in front of the last scores
+            assert N.lib().mdc_test_stages_on_their_way(past, 0, groups, n_tiles, out) == 0
+            assert loaded == awaited and not set(range(out[0], out[1], groups))
