@@ -194,6 +194,79 @@ def test_decode_layer_cp1_matches_oracle(B, S, K, bpc, qpath, exact, dynamic):
         assert (layer.out_lse[b].cpu() - l).abs().max() < 1e-3
 
 
+@pytest.mark.parametrize("fmt,P,d_qk,threshold", [
+    ("mxfp4", 128, 576, True), ("mxfp4", 128, 576, False), ("nvfp4", 128, 576, True), ("nvfp4", 128, 576, False),
+    ("nvfp4", 64, 576, False), ("nvfp4", 64, 512, True)])
+def test_decode_layer_of_every_page_format(fmt, P, d_qk, threshold):
+    """The persistent kernel's other forms of the indexer and attention: chunks of fewer and more stages than its three groups and
+    six ring slots hold; the selection against the top-k of the kernel's own scores, bit for bit, the attention against the oracle."""
+    from dsa_inputs import indexer_case
+    from mega_dsa_cp_b200.layer import DsaDecodeLayer, LayerInputs
+    from mega_dsa_cp_b200.tiles.logits import run_fp4_paged_mqa_logits
+    from oracle import dsa_oracle as orc
+
+    B, K, H, pages = 3, 512, 128, 6016 // P   # (47 stages of 128 tokens, two chunks of 16 and one of 15 without the row threshold)
+    S = pages * P
+    case = indexer_case(B, S, P, fmt, seed=71)
+    g = torch.Generator().manual_seed(72)
+    q_mla = (torch.randn(B, 1, H, d_qk, generator=g) * 0.5).bfloat16()
+    kv = (torch.randn(B * S, 1, d_qk, generator=g) * 0.5).bfloat16()
+    seq = torch.tensor([S, S - 77, K // 2 + 1], dtype=torch.int32)
+    layer = DsaDecodeLayer(B, top_k=K, d_qk=d_qk, fmt=fmt, page_tokens=P, max_pages=pages, blocks_per_chunk=2048 // P, kv_seq_stride=S,
+                           out_dtype=torch.float32, n_ctas=12, row_threshold=threshold)
+    d = lambda t: t.to(DEV)
+    layer.bind(LayerInputs(d(case["fused"]), d(case["bt"]), d(seq), d(case["q"]), d(case["w"]), d(q_mla), d(kv)))
+    logits = torch.zeros(B, S, device=DEV)
+    run_fp4_paged_mqa_logits(d(case["fused"]), d(case["q"]), None, d(case["w"]), d(case["bt"]), logits, 2048 // P, fmt=fmt, page_tokens=P)
+    ref = orc.ref_logits(case["q_deq"], case["w"], case["fused"], case["bt"], 1, fmt=fmt, page_tokens=P)
+    assert torch.allclose(logits.cpu(), ref, rtol=1e-3, atol=1e-4)   # test_logits_vs_oracle's bound
+    for _ in range(2):
+        layer.step()
+        torch.cuda.synchronize()
+        layer.check_status()
+        for b in range(B):
+            ev, ei = orc.local_topk_ref(logits[b].cpu(), 0, S, int(seq[b]), K, 1, 0)
+            n = int(layer.sel_c[b])
+            assert n == ei.numel() and torch.equal(layer.sel_i[b, :n].cpu(), ei), b
+            assert torch.equal(layer.sel_v[b, :n].cpu().view(torch.int32), ev.view(torch.int32)), b
+            o, l = orc.attend_selected_ref(q_mla[b, 0].float(), kv[b * S:(b + 1) * S, 0].float(), ei, 1 / math.sqrt(d_qk))
+            assert (layer.out[b].cpu() - o).abs().max() < 2e-2   # test_decode_layer_cp1_matches_oracle's bounds
+            assert (layer.out_lse[b].cpu() - l).abs().max() < 1e-3
+
+
+@pytest.mark.parametrize("fmt,P,threshold", [("nvfp4", 64, True), ("nvfp4", 64, False), ("nvfp4", 128, True), ("mxfp4", 128, True)])
+def test_layer_step_reports_an_unusable_page(fmt, P, threshold):
+    """A page table entry behind the pool: the step ends within its wait budget with the entry in the status, and a layer on a
+    whole table runs afterwards."""
+    from dsa_inputs import indexer_case
+    from mega_dsa_cp_b200 import _native as N
+    from mega_dsa_cp_b200.layer import DsaDecodeLayer, LayerInputs
+
+    B, S, K, H, DQK = 2, 4096, 512, 128, 576
+    case = indexer_case(B, S, P, fmt, seed=73)
+    g = torch.Generator().manual_seed(74)
+    d = lambda t: t.to(DEV)
+    q_mla, kv = (torch.randn(B, 1, H, DQK, generator=g) * 0.5).bfloat16(), (torch.randn(B * S, 1, DQK, generator=g) * 0.5).bfloat16()
+    outs = []
+    for bad in (False, True, False):
+        bt = case["bt"].clone()
+        if bad:
+            bt[1, S // P // 2] = case["fused"].shape[0]
+        layer = DsaDecodeLayer(B, top_k=K, fmt=fmt, page_tokens=P, max_pages=S // P, blocks_per_chunk=1024 // P, kv_seq_stride=S,
+                               out_dtype=torch.float32, n_ctas=32, row_threshold=threshold)
+        layer.bind(LayerInputs(d(case["fused"]), d(bt), torch.full((B,), S, dtype=torch.int32, device=DEV), d(case["q"]), d(case["w"]),
+                               d(q_mla), d(kv)))
+        layer.step(wait_budget_ns=50_000_000)
+        torch.cuda.synchronize()
+        if bad:
+            st = layer.status.tolist()
+            assert st[0] == N.DEV_BAD_INDEX and st[2:4] == [case["fused"].shape[0], S // P // 2], st
+        else:
+            layer.check_status()
+            outs.append((layer.sel_i.clone(), layer.out.clone()))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
 def test_layer_steps_replay_from_a_cuda_graph():
     """The phase counter lives on the device and the kernel advances it, so a model step -- here 61
     layer-calls, the reference's count (docs/overview.md:10) -- captured once as a CUDA graph replays

@@ -100,6 +100,52 @@ def test_logits_stages_of_the_groups(fmt, P, T, q_fp4, stages):
     assert torch.allclose(got, ref, rtol=1e-3, atol=1e-4), (got - ref).abs().max()   # test_logits_vs_oracle's bound
 
 
+@pytest.mark.parametrize("fmt,P,T,K,bpc,S", [
+    ("nvfp4", 64, 1, 512, 32, 8192),     # keys with their histogram; a stage holds two pages
+    ("nvfp4", 64, 2, 1024, 192, 12288),  # two query tokens on a chunk too long for histograms: scores
+    ("nvfp4", 128, 1, 512, 16, 8192),
+    ("mxfp4", 128, 2, 512, 16, 8192),
+    ("nvfp4", 128, 1, 1024, 16, 1152),   # fewer usable positions than top_k: the -inf of unusable pages is selected too
+])
+def test_unusable_pages_in_every_mode(fmt, P, T, K, bpc, S):
+    """Pages that are missing (-1) or behind the pool, first loads of the ring and refills, one and both of a stage: written
+    scores, chunk lists and row mode give their tokens -inf, and every other token what a call on whole tables gives."""
+    from mega_dsa_cp_b200 import _native as N
+    from mega_dsa_cp_b200.tiles.logits import run_fp4_paged_mqa_logits
+
+    B, pages = 2, S // P
+    case = indexer_case(B, S, P, fmt, q_len=T, q_fp4=(fmt == "mxfp4"), seed=91)
+    want = _run_logits(case, bpc).view(B, T, pages, P)
+    ref = _oracle_logits(case).view(B, T, pages, P)
+    assert torch.allclose(want, ref, rtol=1e-3, atol=1e-4)   # test_logits_vs_oracle's bound
+    bad = torch.tensor([0, pages // 2, pages // 2 + 1, pages - 1])
+    case["bt"][1, bad] = torch.tensor([-1, -7, B * pages, 2**31 - 1], dtype=torch.int32)
+    want[1, :, bad] = float("-inf")
+    want = want.view(B * T, S)
+    d = lambda x: None if x is None else x.to(DEV)
+    row_bpc, n_chunks = min(bpc, 8192 // P), -(-pages // bpc)
+    got = torch.full((B * T, S), float("nan"), device=DEV)
+    cv, ci = torch.zeros(B, T, n_chunks, K, device=DEV), torch.zeros(B, T, n_chunks, K, dtype=torch.int32, device=DEV)
+    rv, ri = torch.zeros(B, T, K, device=DEV), torch.zeros(B, T, K, dtype=torch.int32, device=DEV)
+    cc, rc = torch.zeros(B, T, n_chunks, dtype=torch.int32, device=DEV), torch.zeros(B, T, dtype=torch.int32, device=DEV)
+    for args, kw in (((got, bpc), {}), ((None, bpc), dict(cand_v=cv, cand_i=ci, cand_c=cc, top_k=K)),
+                     ((None, row_bpc), dict(top_k=K, row_topk=(rv, ri, rc)))):
+        status = torch.zeros(8, dtype=torch.int32, device=DEV)
+        run_fp4_paged_mqa_logits(d(case["fused"]), d(case["q"]), d(case["q_sf"]), d(case["w"]), d(case["bt"]), *args, window_exclude=0,
+                                 fmt=fmt, page_tokens=P, status=status, **kw)
+        torch.cuda.synchronize()
+        assert status[0].item() == N.DEV_BAD_INDEX, status.tolist()
+    assert torch.equal(got.cpu(), want)
+    for b in range(B):
+        for t in range(T):
+            row = want[b * T + t]
+            lists = [(c * bpc * P, cv[b, t, c], ci[b, t, c], cc[b, t, c], bpc * P) for c in range(n_chunks)]
+            for lo, v, i, n, size in lists + [(0, rv[b, t], ri[b, t], rc[b, t], S)]:
+                ev, ei = orc.local_topk_ref(row, lo, min(lo + size, S), S, K, 1, 0)
+                assert int(n) == ei.numel() and torch.equal(i[:int(n)].cpu(), ei), (b, t, lo)
+                assert torch.equal(v[:int(n)].cpu().view(torch.int32), ev.view(torch.int32)), (b, t, lo)
+
+
 @pytest.mark.parametrize("fmt,P,T,K,bpc,S,seq,wex", [
     ("mxfp4", 128, 2, 512, 32, 8192, 8192, 128),   # the reference's fused test
     ("mxfp4", 128, 2, 1024, 32, 8192, 8000, 128),
