@@ -116,38 +116,6 @@ __device__ inline void mbar_arrive_if(uint64_t* bar, bool pred) {
                : "memory");
 }
 
-// Shared-memory progress counters (cheaper to poll than an mbarrier for a
-// thread that sits on the tensor-core issue path): release increment, acquire load.
-__device__ inline void red_release_cta_shared_inc(uint32_t* p) {
-  asm volatile("red.release.cta.shared::cta.add.u32 [%0], 1;" ::"r"(smem_u32(p)) : "memory");
-}
-__device__ inline void red_release_cta_shared_inc_if(uint32_t* p, bool pred) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %1, 0;\n @p red.release.cta.shared::cta.add.u32 [%0], 1;\n}" ::"r"(
-                   smem_u32(p)),
-               "r"(static_cast<uint32_t>(pred))
-               : "memory");
-}
-__device__ inline uint32_t ld_acquire_cta_shared_u32(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
-  return v;
-}
-// Bounded wait until a shared counter reaches `target` (same give-up rules as mbar_wait).
-__device__ inline bool counter_wait(const uint32_t* p, uint32_t target, long long budget = (1ll << 31),
-                                    const volatile uint32_t* abort_flag = nullptr) {
-  if (ld_acquire_cta_shared_u32(p) >= target) return true;
-  const long long t0 = clock64();
-  do {
-#pragma unroll 1
-    for (int i = 0; i < 64; ++i) {
-      __nanosleep(20);  // a hot spin would take issue slots from the warps this one waits for
-      if (ld_acquire_cta_shared_u32(p) >= target) return true;
-    }
-    if (abort_flag && *abort_flag) return false;
-  } while (clock64() - t0 < budget);
-  return false;
-}
-
 // 1-D bulk copy global -> shared, completion counted on an mbarrier.  Both
 // addresses 16-byte aligned, size a multiple of 16.
 __device__ inline void bulk_g2s(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {

@@ -808,9 +808,8 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_kernel(const __grid_cons
   const EventSet ev{static_cast<unsigned char*>(p.events.base), p.events.offsets, p.events.my_rank, p.events.world};
   const mdc_layer_params& L = p.layer;
 
-  // Across a task's body only the position of its entry is kept: the rest is read again from shared memory and from the
-  // parameters.  The tiles are functions of their own, and every register that is live across the call is one they
-  // cannot use.
+  // Across a task's body, inlined or called, only the position of its entry is kept: the rest is read again from shared
+  // memory and from the parameters, since the tiles need every register that would be live across them.
   auto cursor = [&]() {
     Cursor c;
     c.row = staged ? sh.row : row_g;
@@ -886,7 +885,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_kernel(const __grid_cons
       }
     }
     __syncthreads();
-    pos = dyn ? pull() : pos + 4 + t.n_waits + t.n_notifies;
+    pos = dyn ? pull() : cur.next_pos(t);
   }
   if (dyn && tid == 0) {   // the last block to finish rewinds the counters for the next launch
     __threadfence();

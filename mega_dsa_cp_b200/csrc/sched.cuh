@@ -45,7 +45,7 @@ struct Cursor {
     t.pos = pos;
     return t;
   }
-  __device__ TaskInfo advance(const TaskInfo& t) const { return read(t.pos + 4 + t.n_waits + t.n_notifies); }
+  __device__ int next_pos(const TaskInfo& t) const { return t.pos + 4 + t.n_waits + t.n_notifies; }
   // dynamic trip-count bound of the task (0 when it has none)
   __device__ int extent(const TaskInfo& t) const {
     return t.extent_src ? static_cast<int>(scalars[t.extent_src] & 0xffffffffull) : 0;

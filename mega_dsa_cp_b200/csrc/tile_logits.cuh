@@ -24,14 +24,16 @@
 // triple the shared-memory traffic of a kernel that has to sustain one stage
 // per ~400 cycles to follow HBM.
 //
-// What bounds the loop is latency between dependent steps and instruction fetch, with every pipe half used (ALU, shared
+// What bounds the loop is latency between dependent steps, with every pipe half used (ALU, shared
 // memory, issue slots and tensor core each need 250-400 cycles per stage).  So the groups share nothing: no counters or
 // barriers between producer and consumer warps, no warp that only polls; a group's step waits for its raw stage and for
 // its own product, both of which have had most of a step to complete.  The form before had two decode groups, two gate
 // groups, two issue warps and a copy warp (one gate group and one issue warp in the persistent kernel), handing stages on
 // in pairs.  32 x 32768 tokens with row top-k 38.9 -> 36.0 us, 37 sequences x 16384 tokens, logits out, 18.0 -> 15.4,
-// two query tokens, 16 x 32768 MXFP4, 32.2 -> 28.8, 3 x 20032 6.4 -> 5.1 (of which the query's loads in flight together
-// 1.0), the persistent kernel's step of 8 x 131072 85.5 -> 76.3 with what else changed there.
+// two query tokens, 16 x 32768 MXFP4, 32.2 -> 28.8, 3 x 20032 6.4 -> 5.1, the persistent kernel's step of 8 x 131072
+// 85.5 -> 76.3: with the query's loads in flight together and the page table read ahead of the length, which shortened the
+// prologue from 6400 to 2570 cycles by clock stamps (1.95 us of the first figure's 2.9, 1.0 of the fourth's), and in the
+// persistent kernel with what else changed there.
 // Three groups with issue and copy warps between them: 43.5 for the
 // first of these; the warps of a group taking turns to issue: 37.7.
 //
