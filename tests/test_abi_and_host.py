@@ -459,14 +459,13 @@ def test_ctypes_mirrors_match_the_header_layout(tmp_path):
             assert int(got[f"{cname}.{fname}"]) == getattr(mirror, fname).offset, (cname, fname)
 
 
-def test_lse_merge_tasks_stay_within_a_wave_and_cover_the_heads():
+def test_lse_merge_tasks_per_sequence():
+    """The count at each boundary of the rule, and the tasks that a layer of that count queues."""
     from mega_dsa_cp_b200.layer import build_layer_dag, lse_groups_for
 
-    for owned in (1, 8, 14, 15, 18, 19, 37, 38, 74, 200):
-        g = lse_groups_for(owned, 148)
-        assert g == 2 or owned * g <= 148
-        per = -(-128 // g)
-        assert sorted(h for q in range(g) for h in range(q * per, min(128, (q + 1) * per))) == list(range(128))
+    for n_ctas, want in ((148, {1: 10, 14: 10, 15: 5, 29: 5, 30: 4, 37: 4, 38: 3, 49: 3, 50: 2, 74: 2, 75: 2, 200: 2}),
+                         (12, {1: 10, 2: 5, 3: 4, 4: 3, 5: 2, 7: 2})):
+        assert {owned: lse_groups_for(owned, n_ctas) for owned in want} == want
     tasks, _, ops = build_layer_dag(3, 4, 1, lse_groups=4)
     from mega_dsa_cp_b200 import _native as N
     assert [t.coords for t in tasks if ops[t.name] == N.OP_LSE_MERGE] == [(b, q, 4) for b in range(3) for q in range(4)]

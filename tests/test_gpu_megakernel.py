@@ -194,10 +194,10 @@ def test_decode_layer_cp1_matches_oracle(B, S, K, bpc, qpath, exact, dynamic):
         assert (layer.out_lse[b].cpu() - l).abs().max() < 1e-3
 
 
-@pytest.mark.parametrize("fmt,P,d_qk,threshold", [
-    ("mxfp4", 128, 576, True), ("mxfp4", 128, 576, False), ("nvfp4", 128, 576, True), ("nvfp4", 128, 576, False),
-    ("nvfp4", 64, 576, False), ("nvfp4", 64, 512, True)])
-def test_decode_layer_of_every_page_format(fmt, P, d_qk, threshold):
+@pytest.mark.parametrize("fmt,P,d_qk,threshold,n_ctas", [   # (n_ctas: 5, 3, 10, 2, 4 and 5 LSE_MERGE tasks per sequence)
+    ("mxfp4", 128, 576, True, 15), ("mxfp4", 128, 576, False, 9), ("nvfp4", 128, 576, True, 30), ("nvfp4", 128, 576, False, 6),
+    ("nvfp4", 64, 576, False, 12), ("nvfp4", 64, 512, True, 15)])
+def test_decode_layer_of_every_page_format(fmt, P, d_qk, threshold, n_ctas):
     """The persistent kernel's other forms of the indexer and attention: chunks of fewer and more stages than its three groups and
     six ring slots hold; the selection against the top-k of the kernel's own scores, bit for bit, the attention against the oracle."""
     from dsa_inputs import indexer_case
@@ -213,7 +213,7 @@ def test_decode_layer_of_every_page_format(fmt, P, d_qk, threshold):
     kv = (torch.randn(B * S, 1, d_qk, generator=g) * 0.5).bfloat16()
     seq = torch.tensor([S, S - 77, K // 2 + 1], dtype=torch.int32)
     layer = DsaDecodeLayer(B, top_k=K, d_qk=d_qk, fmt=fmt, page_tokens=P, max_pages=pages, blocks_per_chunk=2048 // P, kv_seq_stride=S,
-                           out_dtype=torch.float32, n_ctas=12, row_threshold=threshold)
+                           out_dtype=torch.float32, n_ctas=n_ctas, row_threshold=threshold)
     d = lambda t: t.to(DEV)
     layer.bind(LayerInputs(d(case["fused"]), d(case["bt"]), d(seq), d(case["q"]), d(case["w"]), d(q_mla), d(kv)))
     logits = torch.zeros(B, S, device=DEV)
