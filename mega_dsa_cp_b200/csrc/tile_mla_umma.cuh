@@ -168,8 +168,9 @@ __device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, in
   static_assert(S >= 3 && SM::kPanels * kMuHeads * 128 <= (S - 1) * SM::kStageBytes,
                 "two tiles are held while the next is gathered, and the staged query must fit the KV ring behind its first stage");
   constexpr long long kBudget = 1ll << 31;
-  // Warps of a lane quadrant that move the query into tensor memory: the softmax warp and, stand-alone, two gather warps (32 rows x
-  // 2048 slots 49.0 -> 48.1 us; inside the persistent kernel the three of them gained nothing).
+  // Warps of a lane quadrant that move the query into tensor memory: the softmax warp and, stand-alone, two gather warps (3 rows x
+  // 700 slots with window 16.6 -> 16.4 us, 32 x 2048 56.2 -> 55.7, e4m3 16 x 640 17.25 -> 17.1 on one box; on another the last two
+  // are inside the spread.  Inside the persistent kernel the three of them gained nothing).
   constexpr int kMovers = ALONE ? 3 : 1;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned char* kst = smem + SM::kK;
