@@ -167,7 +167,7 @@ __device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, in
   static_assert(kPCol + kMuTile * ESZ / 4 <= 512, "tensor memory over-subscribed");
   static_assert(S >= 3 && SM::kPanels * kMuHeads * 128 <= (S - 1) * SM::kStageBytes,
                 "two tiles are held while the next is gathered, and the staged query must fit the KV ring behind its first stage");
-  constexpr long long kBudget = 1ll << 31;
+  constexpr long long kBudget = 1ll << 31, kDrain = 1ll << 24;   // clock cycles a role waits before it gives up, and after
   // Warps of a lane quadrant that move the query into tensor memory: the softmax warp and, stand-alone, two gather warps (3 rows x
   // 700 slots with window 16.6 -> 16.4 us, 32 x 2048 56.2 -> 55.7, e4m3 16 x 640 17.25 -> 17.1 on one box; on another the last two
   // are inside the spread.  Inside the persistent kernel the three of them gained nothing).
@@ -224,12 +224,15 @@ __device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, in
     report_failure(p.status, MDC_DEV_COPY_TIMEOUT, 16 + what, idx, 0, 0);
     *abort_flag = 1;
   };
+  // The lanes of a warp may have seen the last poll of a wait that ran out differently, and what follows takes whole warps.  So no
+  // lane leaves its role alone: the issue warps vote on every wait, the others go on to the end (of the flag's making, no wait lasts
+  // any more) and write no result.
 
   // Query rows -> tensor memory (16 columns per store), from the copy the gather warps staged
   // in the (still empty) stages 1.. of the KV ring as panels of 128 rows x 128 bytes, 128-byte swizzle.  Mover
   // `m` of its lane quadrant (a warp's number % 4) takes every kMovers-th 16 columns.
   auto query_to_tmem = [&](int m) {
-    if (!mbar_wait(qs_ready, 0, kBudget, abort_flag) && lane == 0) give_up(7, 0);
+    if (!mbar_wait(qs_ready, 0, kBudget, abort_flag)) give_up(7, 0);
     const int row = (warp & 3) * 32 + lane;
     const uint32_t t_row = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
 #pragma unroll 2
@@ -266,9 +269,8 @@ __device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, in
     bool ok = true;
     for (int i = 0; i < n_my; ++i) {
       if (!mbar_wait(s_ready, i & 1, kBudget, abort_flag)) {
-        if (lane == 0) give_up(0, i);
+        if (ok) give_up(0, i);
         ok = false;
-        break;
       }
       umma::fence_after_sync();
       float sv[kMuTile];
@@ -338,9 +340,8 @@ __device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, in
       if (i > 0) {
         // P V of tile i - 1 has read P, and the accumulator holds the tiles up to it, once it has freed its stage
         if (!mbar_wait(&free_[(i - 1) % S], ((i - 1) / S) & 1, kBudget, abort_flag)) {
-          if (lane == 0) give_up(9, i);
+          if (ok) give_up(9, i);
           ok = false;
-          break;
         }
         umma::fence_after_sync();
         if (__any_sync(0xffffffffu, grow)) {
@@ -372,12 +373,12 @@ __device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, in
       __syncwarp();
       mbar_arrive_if(p_ready, lane == 0);
     }
-    if (ok && n_my > 0 && !mbar_wait(o_final, 0, kBudget, abort_flag)) {
-      if (lane == 0) give_up(1, n_my);
+    if (n_my > 0 && !mbar_wait(o_final, 0, kBudget, abort_flag)) {
+      if (ok) give_up(1, n_my);
       ok = false;
     }
     umma::fence_after_sync();
-    if (ok) {
+    if (__all_sync(0xffffffffu, ok)) {
       const bool live = l > 0.f;
       const float inv = live ? p.output_scale / l : 0.f;
       const float lse = live ? log2f(l) + c2 * m_used : neg_inf;
@@ -458,7 +459,6 @@ __device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, in
   } else if (warp >= kMuGatherWarp0 && warp < kMuGatherWarp0 + kMuGatherWarps) {
     // ---------------- gather warps: 8 rows of every tile each, up to two tiles in flight per warp
     const int gw = warp - kMuGatherWarp0;
-    bool ok = true;
     // Row pointers are looked up four tiles at a time and a batch ahead: a page-table read takes about as
     // long as a whole tile, and one tile of lead left it on the path (42 against 83 GB/s per SM in a copy of
     // this loop with 8 warps and rows that four blocks share).
@@ -496,10 +496,7 @@ __device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, in
       mbar_arrive_if(qs_ready, lane == 0);
       if constexpr (ALONE) query_to_tmem(warp / 4);
       // stages 1.. are free for KV tiles once all of them have moved their share
-      if (!mbar_wait(q_ready, 0, kBudget, abort_flag)) {
-        if (lane == 0) give_up(8, 0);
-        ok = false;
-      }
+      if (!mbar_wait(q_ready, 0, kBudget, abort_flag)) give_up(8, 0);
     }
     // Tiles [done, i) have been issued but not yet published.  A tile is published as soon as
     // its copies have landed -- never held back until the NEXT tile could be issued: when the
@@ -512,11 +509,11 @@ __device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, in
       for (int t = done; t < upto; ++t) mbar_arrive_if(&full[t % S], lane == 0);
       done = upto;
     };
-    if (i0 == 1 && ok) {  // tile 0 was issued before the query hand-over: it has had time to land, publish it now
+    if (i0 == 1) {  // tile 0 was issued before the query hand-over: it has had time to land, publish it now
       cp_async_wait<0>();
       publish(1);
     }
-    for (int i = i0; i < n_my && ok; ++i) {
+    for (int i = i0; i < n_my; ++i) {
       const int j = i % kMuBatch;   // tile i's place in the batch of row pointers
       if (j == 0) {
         cur = nxt;
@@ -530,11 +527,7 @@ __device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, in
             cp_async_wait<0>();
             publish(i);
           }
-          if (!mbar_wait(&free_[st], par, kBudget, abort_flag)) {
-            if (lane == 0) give_up(2, i);
-            ok = false;
-            break;
-          }
+          if (!mbar_wait(&free_[st], par, kBudget, abort_flag)) give_up(2, i);
         }
       }
       const uint32_t bits = mla_umma_gather_rows<ROWB>(p, cur, j, kst + st * SM::kStageBytes, gw, lane);
@@ -545,18 +538,19 @@ __device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, in
       }
     }
     cp_async_wait<0>();
-    if (ok && n_my > 0) publish(n_my);
+    if (n_my > 0) publish(n_my);
   } else if (warp == kMuIssueWarp) {
     // ---------------- S = Q K^T of tile i, once it is gathered and the softmax warps have taken tile i - 1
     constexpr uint32_t idesc_qk = umma::idesc_mla(FP8, kMuHeads, kMuTile, false);
     const uint32_t kst_u = smem_u32(kst);
     bool ok = mbar_wait(q_ready, 0, kBudget, abort_flag);
-    if (!ok && lane == 0) give_up(3, 0);
+    if (!ok) give_up(3, 0);
     for (int i = 0; i < n_my; ++i) {
       ok = ok && mbar_wait(&full[i % S], (i / S) & 1, kBudget, abort_flag) &&
            (i == 0 || mbar_wait(s_taken, (i - 1) & 1, kBudget, abort_flag));
       if (!__all_sync(0xffffffffu, ok)) {
         if (lane == 0) give_up(4, i);
+        if (i > 0) mbar_wait(s_ready, (i - 1) & 1, kDrain);   // the last product (without the block's flag)
         break;
       }
       umma::fence_after_sync();
@@ -580,6 +574,7 @@ __device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, in
       ok = __all_sync(0xffffffffu, mbar_wait(p_ready, i & 1, kBudget, abort_flag));
       if (!ok) {
         if (lane == 0) give_up(5, i);
+        for (int j = max(0, i - S); j < i; ++j) mbar_wait(&free_[j % S], (j / S) & 1, kDrain);   // the last products
         break;
       }
       umma::fence_after_sync();
@@ -600,8 +595,8 @@ __device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, in
       // them here, or one could land after the barriers are invalidated below, on shared memory
       // that the block's next task already uses for something else.
       for (int i = max(0, n_my - S); i < n_my; ++i) {
-        if (!mbar_wait(&free_[i % S], (i / S) & 1, kBudget, abort_flag)) {
-          if (lane == 0) give_up(6, i);
+        if (!mbar_wait(&free_[i % S], (i / S) & 1, kBudget)) {   // (also when another role has given up)
+          give_up(6, i);
           break;
         }
       }
