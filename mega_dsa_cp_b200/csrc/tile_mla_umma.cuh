@@ -225,8 +225,8 @@ __device__ __forceinline__ void mla_umma_tile(const mdc_sparse_mla_params& p, in
     *abort_flag = 1;
   };
   // The lanes of a warp may have seen the last poll of a wait that ran out differently, and what follows takes whole warps.  So no
-  // lane leaves its role alone: the issue warps vote on every wait, the others go on to the end (of the flag's making, no wait lasts
-  // any more) and write no result.
+  // lane leaves its role alone: the issue warps vote on every wait, the others go on to the end (once the flag is set no
+  // wait lasts) and write no result.
 
   // Query rows -> tensor memory (16 columns per store), from the copy the gather warps staged
   // in the (still empty) stages 1.. of the KV ring as panels of 128 rows x 128 bytes, 128-byte swizzle.  Mover
